@@ -8,12 +8,17 @@
 //   MinP                :130-146
 //   RepetitionPenalty   :160-181
 //   MultinomialSampler  crates/decode/src/sampler.rs:31-58  (the uniform draw is an input)
-// The reference sorts the whole vocabulary per step for TopK / TopP; here a row is one CTA that finds
-// the cut by a radix select over an order-preserving integer key of the logit, four bits per pass:
-// every thread keeps its own 16 bins (count, probability mass) in shared memory (no atomics, a fixed
-// summation order: results do not change between runs), the bins are reduced across the block, and one
-// thread walks them from the top. Ties at the cut are kept in index order, as the reference's stable
-// sort does.
+// The reference sorts the whole vocabulary per step for TopK / TopP; here the cut is found by a radix select over an
+// order-preserving integer key of the logit, 11 bits per pass (three passes of 2048 bins). One CTA per row left most of the
+// chip idle; a row is a cluster of eight CTAs that meet through each other's shared memory (rows below kClusterFrom
+// values: one CTA). What bounds them is the work that does not shrink with the slice, barriers and the reduction of the
+// bins, so a CTA has 256 threads (64 x 151936, TopK: 47 us; 512 threads 57, 1024 threads with the slice held in
+// shared memory 75) and goes over its slice as rarely as it can: values that can still hold the cut, or all that TopK has left,
+// are listed in shared memory, and later passes go over the list. Bins hold integers, counts and probabilities in units of
+// 2^-(24 + lo_bits), so shared-memory atomics give the same sums in any order and results do not change between runs. Ties
+// at the cut are kept in index order, as the reference's stable sort does.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "logismos_kernels.h"
 
@@ -21,9 +26,17 @@ namespace {
 
 using namespace lg;
 
-constexpr int kThreads = 1024;
-constexpr int kBins = 16;
-constexpr size_t kSelectSmem = (size_t)kBins * kThreads * 8 + 1024;
+namespace cg = cooperative_groups;
+
+constexpr int kThreads = 256;
+constexpr int kBins = 2048;       // 11 bits of the key
+constexpr int kMaxCluster = 8;    // portable cluster size
+constexpr int kSegment = kBins / kMaxCluster;
+static_assert(kSegment == kThreads, "a thread per bin of a segment");
+// Below this a CTA's share of a row is one load per thread and the cluster's barriers cost more than they save (top-p of 64
+// rows: 2500 values 24 us either way, 4001 28 as one CTA and 27 as a cluster, 8000 42 and 31).
+constexpr int kClusterFrom = 2048;
+constexpr int kListed = 1024;     // values that a CTA can list
 
 // larger float <-> larger key; NaN is ordered like -inf (TopK folds NaN to -inf before its sort)
 LG_DEVINL uint32_t order_key(float v) {
@@ -32,9 +45,20 @@ LG_DEVINL uint32_t order_key(float v) {
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-__global__ void temperature_kernel(float* __restrict__ logits, int64_t total, float t) {
+// a true division, as the reference does (not a reciprocal multiply); four values per thread where the pointer is aligned
+__global__ void temperature_kernel(float* __restrict__ logits, int64_t total, float t, int vec) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < total) logits[i] = logits[i] / t;  // a true division, as the reference does (not a reciprocal multiply)
+  if (!vec) {
+    if (i < total) logits[i] = logits[i] / t;
+    return;
+  }
+  if (4 * i + 4 <= total) {
+    float4 v = reinterpret_cast<float4*>(logits)[i];
+    v.x /= t; v.y /= t; v.z /= t; v.w /= t;
+    reinterpret_cast<float4*>(logits)[i] = v;
+  } else {
+    for (int64_t j = 4 * i; j < total; ++j) logits[j] = logits[j] / t;
+  }
 }
 
 // one thread per row walks the row's list in order: a token listed twice is penalised twice
@@ -52,267 +76,474 @@ __global__ void repetition_penalty_rows_kernel(float* __restrict__ logits, int r
   }
 }
 
-// block-wide maximum and sum of exp(l - max); finite_only: non-finite logits carry no mass (the sampler)
-LG_DEVINL void row_max_sum(const float* __restrict__ l, int n, bool finite_only, float* red, float& mx, float& sum) {
+// What the CTAs of a row tell each other, and the values [begin, end) of the row that this CTA owns.
+struct Shared {
+  float max[kMaxCluster], sum[kMaxCluster];
+  unsigned long long seg[kMaxCluster], above;  // above: of the last radix pass, as are bin and none
+  uint32_t bin, none;
+  uint32_t tie_counts[kMaxCluster];
+  uint32_t best, count;
+  float red[32];
+};
+
+struct Row {
+  float* l;
+  int n, begin, end, rank, size;
+  bool vec;  // the row is 16-byte aligned
+  const int2* list = nullptr;  // (index, value) of the values that `each` and `mask` go over instead of the slice
+  int listed = 0;
+
+  LG_DEVINL Row(float* logits, int n_, const cg::cluster_group& c) : n(n_) {
+    rank = (int)c.block_rank();
+    size = (int)c.num_blocks();
+    l = logits + (size_t)(blockIdx.x / size) * n;
+    const int per = ((n + size - 1) / size + 3) & ~3;
+    begin = min(rank * per, n);
+    end = min(begin + per, n);
+    vec = (reinterpret_cast<uintptr_t>(l) & 15) == 0;
+  }
+
+  // f(index, value) for every value of the slice, whichever thread it falls to
+  template <typename F>
+  LG_DEVINL void stream(F&& f) const {
+    if (vec) {
+      const int full = begin + ((end - begin) & ~3);
+#pragma unroll 4
+      for (int i = begin + 4 * (int)threadIdx.x; i < full; i += 4 * kThreads) {
+        const float4 v = *reinterpret_cast<const float4*>(l + i);
+        f(i, v.x); f(i + 1, v.y); f(i + 2, v.z); f(i + 3, v.w);
+      }
+      for (int i = full + (int)threadIdx.x; i < end; i += kThreads) f(i, l[i]);
+    } else {
+#pragma unroll 4
+      for (int i = begin + (int)threadIdx.x; i < end; i += kThreads) f(i, l[i]);
+    }
+  }
+
+  template <typename F>
+  LG_DEVINL void each(F&& f) const {
+    if (!list) { stream(f); return; }
+    for (int j = threadIdx.x; j < listed; j += kThreads) {
+      const int2 e = list[j];
+      f(e.x, __int_as_float(e.y));
+    }
+  }
+
+  // f(i, v) for the whole slice; the values for which it holds are listed, unless there are more than `room` holds
+  template <typename F>
+  LG_DEVINL void collect(int2* room, uint32_t* count, F&& f) {
+    if (threadIdx.x == 0) *count = 0;
+    __syncthreads();
+    bool open = true;  // until this thread has seen more than the room holds
+    stream([&](int i, float v) {
+      if (!f(i, v) || !open) return;
+      open = *reinterpret_cast<volatile uint32_t*>(count) <= (uint32_t)kListed;
+      if (!open) return;
+      const uint32_t lanes = __activemask(), lane = threadIdx.x & 31;
+      uint32_t at = 0;
+      if (lane == (uint32_t)(__ffs(lanes) - 1)) at = atomicAdd(count, (uint32_t)__popc(lanes));
+      at = __shfl_sync(lanes, at, __ffs(lanes) - 1) + __popc(lanes & ((1u << lane) - 1u));
+      if (at < (uint32_t)kListed) room[at] = make_int2(i, __float_as_int(v));
+    });
+    __syncthreads();
+    if (*count <= (uint32_t)kListed) { list = room; listed = (int)*count; }
+  }
+
+  // the values for which drop(value) holds become -inf; what is -inf already is not written again
+  template <typename F>
+  LG_DEVINL void mask(F&& drop) const {
+    auto one = [&](float& v) {
+      const bool d = v != -INFINITY && drop(v);
+      if (d) v = -INFINITY;
+      return d;
+    };
+    if (!list && vec) {
+      const int full = begin + ((end - begin) & ~3);
+#pragma unroll 4
+      for (int i = begin + 4 * (int)threadIdx.x; i < full; i += 4 * kThreads) {
+        float4 v = *reinterpret_cast<const float4*>(l + i);
+        const bool a = one(v.x), b = one(v.y), c = one(v.z), d = one(v.w);
+        if (a || b || c || d) *reinterpret_cast<float4*>(l + i) = v;
+      }
+      for (int i = full + (int)threadIdx.x; i < end; i += kThreads) {
+        float v = l[i];
+        if (one(v)) l[i] = v;
+      }
+    } else {
+      each([&](int i, float v) { if (one(v)) l[i] = v; });
+    }
+  }
+};
+
+LG_DEVINL void row_sync(const cg::cluster_group& c, const Row& row) {
+  if (row.size == 1) __syncthreads();
+  else c.sync();
+}
+
+// every CTA of the row gets value[r] of each CTA r in its own sh.field[r]; a barrier of the cluster makes it visible
+template <typename T>
+LG_DEVINL void tell(const cg::cluster_group& c, const Row& row, T* field, T value) {
+  if ((int)threadIdx.x < row.size) c.map_shared_rank(field, (int)threadIdx.x)[row.rank] = value;
+}
+
+// The row's maximum and the sum of exp(l - max); finite_only: non-finite logits carry no mass (the sampler). What is
+// above -inf is listed where it fits, unless room is null.
+LG_DEVINL void row_max_sum(const cg::cluster_group& c, Row& row, bool finite_only, int2* room, Shared& sh, float& mx, float& sum) {
   float m = -INFINITY;
-  for (int i = threadIdx.x; i < n; i += kThreads) m = fmaxf(m, l[i]);  // fmaxf ignores NaN, as f32::max does
-  mx = block_max(m, red);
+  if (room) {
+    row.collect(room, &sh.count, [&](int, float v) {
+      m = fmaxf(m, v);  // fmaxf ignores NaN, as f32::max does
+      return !(v == -INFINITY);
+    });
+  } else {
+    row.stream([&](int, float v) { m = fmaxf(m, v); });
+  }
+  tell(c, row, sh.max, block_max(m, sh.red));
+  row_sync(c, row);
+  mx = sh.max[0];
+  for (int r = 1; r < row.size; ++r) mx = fmaxf(mx, sh.max[r]);
   float s = 0.0f;
-  for (int i = threadIdx.x; i < n; i += kThreads) {
-    const float v = l[i];
+  row.each([&](int, float v) {
     const bool fin = fabsf(v) <= 3.402823466e38f;  // false for inf and NaN
-    s += (finite_only && !fin) ? 0.0f : expf(v - mx);
-  }
-  sum = block_sum(s, red);
+    if (!(finite_only && !fin) && v != -INFINITY) s += expf(v - mx);
+  });
+  if (!finite_only && mx == -INFINITY) s = NAN;  // exp(-inf + inf)
+  tell(c, row, sh.sum, block_sum(s, sh.red));
+  row_sync(c, row);
+  sum = 0.0f;
+  for (int r = 0; r < row.size; ++r) sum += sh.sum[r];
 }
 
-// Radix select shared by TopK (by count) and TopP (by probability mass). On return *key_out is the
-// key at which the cut falls, *above_* what lies strictly above it, *ties the number of elements with
-// exactly that key, *none is set when the target was never reached (everything is kept).
+// Radix select shared by TopK (by count) and TopP (by probability mass). Returns the key at which the cut falls and
+// leaves in `sh` what lies strictly above it, and `none` when the target was never reached (everything is kept).
 template <bool BY_MASS>
-LG_DEVINL void radix_select(const float* __restrict__ l, int n, float mx, float inv_sum, float target_mass, uint32_t target_count,
-                            uint8_t* smem, uint32_t& key_out, float& above_mass, uint32_t& above_count, uint32_t& ties, bool& none) {
-  uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);                       // [kBins][kThreads]
-  float* mass = reinterpret_cast<float*>(smem + (size_t)kBins * kThreads * 4);  // [kBins][kThreads]
-  __shared__ uint32_t s_prefix, s_cnt_above, s_ties;
-  __shared__ float s_mass_above;
-  __shared__ int s_none;
-  __shared__ uint32_t r_cnt[kBins];
-  __shared__ float r_mass[kBins];
-  if (threadIdx.x == 0) { s_prefix = 0; s_cnt_above = 0; s_mass_above = 0.0f; s_none = 0; s_ties = 0; }
-  __syncthreads();
-  for (int shift = 28; shift >= 0; shift -= 4) {
-    const uint32_t prefix = s_prefix;
-    const uint32_t pmask = shift == 28 ? 0u : (0xffffffffu << (shift + 4));
-#pragma unroll
-    for (int d = 0; d < kBins; ++d) {
-      cnt[d * kThreads + threadIdx.x] = 0;
-      if (BY_MASS) mass[d * kThreads + threadIdx.x] = 0.0f;
-    }
-    for (int i = threadIdx.x; i < n; i += kThreads) {
-      const float v = l[i];
+LG_DEVINL uint32_t radix_select(const cg::cluster_group& c, Row& row, float mx, float inv_sum, unsigned long long target_mass, uint32_t target_count, int lo_bits,
+                                uint32_t* bins, int2* room, Shared& sh) {
+  uint32_t* cnt = bins;         // BY_MASS: the leading 24 bits of probabilities, and the lo_bits below them
+  uint32_t* lo = bins + kBins;  // (bins without mass cannot hold the cut, so counts of them are not needed)
+  const float unit = ldexpf(1.0f, 24 + lo_bits);
+  const uint32_t lo_mask = (1u << lo_bits) - 1u;
+  uint32_t prefix = 0, cnt_above = 0;
+  unsigned long long mass_above = 0;
+#pragma unroll 1
+  for (int pass = 0; pass < 3; ++pass) {
+    const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
+    const uint32_t pmask = pass == 0 ? 0u : pass == 1 ? 0xffe00000u : 0xfffffc00u;
+    const uint32_t bmask = pass == 2 ? 1023u : 2047u;
+    for (int i = threadIdx.x; i < (BY_MASS ? 2 : 1) * kBins; i += kThreads) bins[i] = 0;
+    if (threadIdx.x == 0) sh.none = 1;
+    if (pass == 1 && !row.list) row.collect(room, &sh.count, [&](int, float v) { return (order_key(v) & pmask) == prefix; });
+    __syncthreads();
+    row.each([&](int, float v) {
       const uint32_t key = order_key(v);
-      if ((key & pmask) != prefix) continue;
-      const int d = (key >> shift) & 15;
-      cnt[d * kThreads + threadIdx.x] += 1;
-      if (BY_MASS) mass[d * kThreads + threadIdx.x] += expf(v - mx) * inv_sum;
-    }
-    __syncthreads();
-    {  // two warps per bin, fixed order
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      const int d = warp >> 1, half = warp & 1;
-      uint32_t c = 0;
-      float m = 0.0f;
-      for (int j = 0; j < kThreads / 64; ++j) {
-        const int t = half * (kThreads / 2) + j * 32 + lane;
-        c += cnt[d * kThreads + t];
-        if (BY_MASS) m += mass[d * kThreads + t];
+      if ((key & pmask) != prefix) return;
+      const uint32_t d = (key >> shift) & bmask;
+      if (!BY_MASS) {
+        atomicAdd(cnt + d, 1u);
+        return;
       }
+      if (!(v > -INFINITY)) return;
+      const unsigned long long m = __float2ull_rn(expf(v - mx) * inv_sum * unit);
+      if (m >> lo_bits) atomicAdd(cnt + d, (uint32_t)(m >> lo_bits));
+      if ((uint32_t)m & lo_mask) atomicAdd(lo + d, (uint32_t)m & lo_mask);
+    });
+    row_sync(c, row);
+    // the bins are summed over the cluster in kMaxCluster segments, one per CTA (or all by the one CTA), and every CTA
+    // gets every segment's total
+    const int own_segs = kMaxCluster / row.size;
+    __shared__ unsigned long long w_seg[kMaxCluster][kThreads / 32];
+    for (int i = 0; i < own_segs; ++i) {
+      const int j = (row.rank + i) * kSegment + threadIdx.x;
+      unsigned long long m = 0;  // count or mass
+      for (int r = 0; r < row.size; ++r) {
+        const uint32_t a = c.map_shared_rank(cnt, r)[j];
+        m += BY_MASS ? ((unsigned long long)a << lo_bits) + c.map_shared_rank(lo, r)[j] : (unsigned long long)a;
+      }
+      // the CTA's own segment, which only it reads from here on: the sums stay where its own addends were
+      cnt[j] = (uint32_t)(BY_MASS ? m >> lo_bits : m);
+      if (BY_MASS) lo[j] = (uint32_t)m & lo_mask;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        c += __shfl_xor_sync(0xffffffffu, c, o);
-        if (BY_MASS) m += __shfl_xor_sync(0xffffffffu, m, o);
-      }
-      __syncthreads();
-      if (lane == 0 && half == 0) { r_cnt[d] = c; r_mass[d] = m; }
-      __syncthreads();
-      if (lane == 0 && half == 1) { r_cnt[d] += c; r_mass[d] += m; }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      int sel = -1;
-      uint32_t ca = s_cnt_above;
-      float ma = s_mass_above;
-      for (int d = kBins - 1; d >= 0; --d) {
-        if (r_cnt[d] == 0) continue;
-        const bool reached = BY_MASS ? (ma + r_mass[d] >= target_mass) : (ca + r_cnt[d] >= target_count);
-        if (reached) { sel = d; break; }
-        ca += r_cnt[d];
-        ma += r_mass[d];
-      }
-      if (sel < 0) {
-        // the target is beyond the total (p above the rounded total mass): everything is kept; at a later
-        // level only rounding can bring us here: settle on the lowest occupied bin
-        if (shift == 28) s_none = 1;
-        ca = s_cnt_above; ma = s_mass_above;
-        for (int d = kBins - 1; d >= 0; --d) {
-          if (r_cnt[d] == 0) continue;
-          sel = d;
-        }
-        for (int d = kBins - 1; d > sel; --d) { ca += r_cnt[d]; ma += r_mass[d]; }
-        if (sel < 0) sel = 0;
-      }
-      s_cnt_above = ca;
-      s_mass_above = ma;
-      s_prefix = prefix | ((uint32_t)sel << shift);
-      s_ties = r_cnt[sel];
+      for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+      if ((threadIdx.x & 31) == 0) w_seg[i][threadIdx.x >> 5] = m;
     }
     __syncthreads();
-    if (s_none) break;
+    if (threadIdx.x < kMaxCluster) {
+      const int i = row.size == 1 ? (int)threadIdx.x : 0;
+      unsigned long long m = 0;
+      for (int w = 0; w < kThreads / 32; ++w) m += w_seg[i][w];
+      c.map_shared_rank(sh.seg, row.size == 1 ? 0 : (int)threadIdx.x)[row.rank + i] = m;
+    }
+    row_sync(c, row);
+    // the segment in which the target is reached, from the top (a later pass lies inside a bin that reached it)
+    const unsigned long long target = BY_MASS ? target_mass : target_count;
+    unsigned long long above = BY_MASS ? mass_above : cnt_above;
+    int sel = -1;
+    for (int r = kMaxCluster - 1; r >= 0; --r) {
+      if (sh.seg[r] == 0) continue;
+      if (above + sh.seg[r] >= target) { sel = r; break; }
+      above += sh.seg[r];
+    }
+    if (sel >= 0 && row.rank == (row.size == 1 ? 0 : sel) && threadIdx.x < 32) {  // 32 bins at a time from the top
+      const int lane = threadIdx.x, first = sel * kSegment;
+      for (int b = kSegment - 32; b >= 0; b -= 32) {
+        const int j = first + b + 31 - lane;  // lane 0 holds the highest
+        const unsigned long long own = BY_MASS ? ((unsigned long long)cnt[j] << lo_bits) + lo[j] : cnt[j];
+        unsigned long long m = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long t = __shfl_up_sync(0xffffffffu, m, o);
+          if (lane >= o) m += t;
+        }
+        const uint32_t hit = __ballot_sync(0xffffffffu, own > 0 && above + m >= target);
+        if (hit) {
+          const int at = __ffs(hit) - 1;
+          const uint32_t bin = (uint32_t)(first + b + 31 - at);
+          const unsigned long long over = above + __shfl_sync(0xffffffffu, m - own, at);
+          if (lane < row.size) {
+            Shared* o = c.map_shared_rank(&sh, lane);
+            o->bin = bin; o->above = over; o->none = 0;
+          }
+          break;
+        }
+        above += __shfl_sync(0xffffffffu, m, 31);
+      }
+    }
+    row_sync(c, row);
+    if (sh.none) return 0;
+    prefix |= sh.bin << shift;
+    if (BY_MASS) mass_above = sh.above;
+    else cnt_above = (uint32_t)sh.above;
+    __syncthreads();  // read by all before the next pass sets it again
   }
-  key_out = s_prefix;
-  above_mass = s_mass_above;
-  above_count = s_cnt_above;
-  ties = s_ties;
-  none = s_none != 0;
+  return prefix;
 }
 
-// Elements with key == cut, in index order: the first `keep_ties` stay. Tiles of the block size, an
-// ordered count across the block per tile.
-LG_DEVINL void mask_below_cut(float* __restrict__ l, int n, uint32_t cut, uint32_t ties, uint32_t keep_ties, bool mask_nan) {
-  if (keep_ties >= ties) {
-    for (int i = threadIdx.x; i < n; i += kThreads) {
-      const float v = l[i];
-      if (order_key(v) < cut || (mask_nan && v != v)) l[i] = -INFINITY;
+// Values below the cut become -inf, and of those with key == cut all but the first `keep` in index order.
+LG_DEVINL void mask_below_cut(const cg::cluster_group& c, const Row& row, uint32_t cut, unsigned long long keep, bool mask_nan, Shared& sh) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ uint32_t s_warp[kThreads / 32];
+  uint32_t base = 0, ties = 0;  // ties in the slices before this one, and in the row
+  if (keep != ~0ull) {
+    uint32_t own = 0;
+    row.each([&](int, float v) { own += order_key(v) == cut ? 1u : 0u; });
+    own = __reduce_add_sync(0xffffffffu, own);
+    if (lane == 0) s_warp[warp] = own;
+    __syncthreads();
+    uint32_t total = 0;
+    for (int w = 0; w < kThreads / 32; ++w) total += s_warp[w];
+    tell(c, row, sh.tie_counts, total);
+    row_sync(c, row);
+    for (int r = 0; r < row.size; ++r) {
+      if (r < row.rank) base += sh.tie_counts[r];
+      ties += sh.tie_counts[r];
     }
+  }
+  if (keep >= ties) {
+    row.mask([&](float v) { return order_key(v) < cut || (mask_nan && v != v); });
     return;
   }
-  __shared__ uint32_t s_warp[kThreads / 32];
-  __shared__ uint32_t s_base;
-  if (threadIdx.x == 0) s_base = 0;
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i0 = 0; i0 < n; i0 += kThreads) {
+  for (int i0 = row.begin; i0 < row.end; i0 += kThreads) {
     const int i = i0 + threadIdx.x;
-    const float v = i < n ? l[i] : 0.0f;
-    const uint32_t key = i < n ? order_key(v) : 0u;
-    const bool tie = i < n && key == cut;
+    const float v = i < row.end ? row.l[i] : 0.0f;
+    const uint32_t key = i < row.end ? order_key(v) : 0u;
+    const bool tie = i < row.end && key == cut;
     const uint32_t bal = __ballot_sync(0xffffffffu, tie);
+    __syncthreads();
     if (lane == 0) s_warp[warp] = __popc(bal);
     __syncthreads();
-    uint32_t before = s_base;
-    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    uint32_t before = base;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (w < warp) before += s_warp[w];
+      base += s_warp[w];
+    }
     const uint32_t rank = before + __popc(bal & ((1u << lane) - 1u));
-    if (i < n && (key < cut || (tie && rank >= keep_ties) || (mask_nan && v != v))) l[i] = -INFINITY;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t t = 0;
-      for (int w = 0; w < kThreads / 32; ++w) t += s_warp[w];
-      s_base += t;
-    }
-    __syncthreads();
+    if (i < row.end && (key < cut || (tie && rank >= keep) || (mask_nan && v != v))) row.l[i] = -INFINITY;
   }
 }
 
-__global__ void __launch_bounds__(kThreads)
+// A CTA may not leave while another still reads its shared memory: every kernel ends with a barrier of the cluster.
+
+// 170 -> 49 us on 64 x 151936, k = 50
+__global__ void __launch_bounds__(kThreads, 4)
 top_k_kernel(float* __restrict__ logits, int n, int k) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  float* l = logits + (size_t)blockIdx.x * n;
-  uint32_t cut, above_c, ties;
-  float above_m;
-  bool none;
-  radix_select<false>(l, n, 0.0f, 0.0f, 0.0f, (uint32_t)k, smem, cut, above_m, above_c, ties, none);
+  __shared__ uint32_t bins[kBins];
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  const cg::cluster_group c = cg::this_cluster();
+  Row row(logits, n, c);
+  row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
+  const uint32_t cut = radix_select<false>(c, row, 0.0f, 0.0f, 0ull, (uint32_t)k, 0, bins, room, sh);
+  row.list = nullptr;
   // every element tied with the k-th largest survives (the reference masks only `l < threshold`)
-  mask_below_cut(l, n, cut, ties, ties, true);
+  mask_below_cut(c, row, cut, ~0ull, true, sh);
+  row_sync(c, row);
 }
 
-__global__ void __launch_bounds__(kThreads)
+// 186 -> 36 us on 64 x 151936 after top-k 50, 215 -> 100 us on whole rows
+__global__ void __launch_bounds__(kThreads, 4)
 top_p_kernel(float* __restrict__ logits, int n, float p) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float red[32];
-  __shared__ uint32_t s_keep;
-  float* l = logits + (size_t)blockIdx.x * n;
+  __shared__ uint32_t bins[2 * kBins];
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  const cg::cluster_group c = cg::this_cluster();
+  Row row(logits, n, c);
+  row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
   float mx, sum;
-  row_max_sum(l, n, false, red, mx, sum);
+  row_max_sum(c, row, false, room, sh, mx, sum);
+  const bool whole = row.list != nullptr;  // the list has all that is above -inf: nothing else is to be masked
   const float inv = sum > 0.0f ? 1.0f / sum : 1.0f;
-  uint32_t cut, above_c, ties;
-  float above_m;
-  bool none;
-  radix_select<true>(l, n, mx, inv, p, 0u, smem, cut, above_m, above_c, ties, none);
-  if (none) return;  // the mass never reaches p: the reference keeps everything
-  if (threadIdx.x == 0) {
-    // the tied elements share one probability; they are taken one by one until the mass reaches p
-    float q = 0.0f;
-    {
+  // sums of the low halves of a slice fit 32 bits
+  const int slice = (n + row.size - 1) / row.size + 4, lo_bits = min(16, __clz(slice) - 1);
+  const float unit = ldexpf(1.0f, 24 + lo_bits);
+  const unsigned long long target = (unsigned long long)ceil((double)p * (double)unit);
+  const bool finite = fabsf(mx) <= 3.402823466e38f;
+  if (finite && !(sum > 0.0f)) {
+    // a NaN took the sum: probabilities stay unnormalised, and the first maximum alone has mass one
+    row.list = nullptr;
+    mask_below_cut(c, row, order_key(mx), 1ull, false, sh);
+  } else if (finite) {  // an infinite maximum leaves no probability that is a number: the mass never reaches p
+    const uint32_t cut = radix_select<true>(c, row, mx, inv, target, 0u, lo_bits, bins, room, sh);
+    if (!sh.none) {  // otherwise the mass never reaches p: the reference keeps everything
+      // the tied elements share one probability; they are taken one by one until the mass reaches p
       const uint32_t b = (cut & 0x80000000u) ? (cut & 0x7fffffffu) : ~cut;
-      q = expf(__uint_as_float(b) - mx) * inv;
+      const unsigned long long q = __float2ull_rn(expf(__uint_as_float(b) - mx) * inv * unit);
+      const unsigned long long missing = target > sh.above ? target - sh.above : 0ull;
+      if (!whole) row.list = nullptr;
+      mask_below_cut(c, row, cut, max((missing + q - 1) / q, 1ull), false, sh);
     }
-    float cum = above_m;
-    uint32_t m = 0;
-    do { cum += q; ++m; } while (cum < p && m < ties);
-    s_keep = m;
   }
-  __syncthreads();
-  mask_below_cut(l, n, cut, ties, s_keep, false);
+  row_sync(c, row);
 }
 
-__global__ void __launch_bounds__(kThreads)
+// 53 -> 39 us on 64 x 151936
+__global__ void __launch_bounds__(kThreads, 4)
 min_p_kernel(float* __restrict__ logits, int n, float p) {
-  __shared__ float red[32];
-  float* l = logits + (size_t)blockIdx.x * n;
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  const cg::cluster_group c = cg::this_cluster();
+  Row row(logits, n, c);
+  row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
   float mx, sum;
-  row_max_sum(l, n, false, red, mx, sum);
+  row_max_sum(c, row, false, room, sh, mx, sum);
   const bool norm = sum > 0.0f;
   const float max_p = norm ? 1.0f / sum : 1.0f;  // exp(0) over the sum
   const float threshold = p * max_p;
-  for (int i = threadIdx.x; i < n; i += kThreads) {
-    float pr = expf(l[i] - mx);
+  row.mask([&](float v) {
+    float pr = expf(v - mx);
     if (norm) pr /= sum;
-    if (pr < threshold) l[i] = -INFINITY;
-  }
+    return pr < threshold;
+  });
+  row_sync(c, row);
 }
 
-// MultinomialSampler::sample for a given uniform draw: thread t owns the contiguous slice
-// [t c, (t + 1) c) of the row; slice masses are scanned across the block and the thread(s) whose slice
-// can hold the draw walk it as the reference does (u < p_i returns i, else u -= p_i).
-__global__ void __launch_bounds__(kThreads)
+// MultinomialSampler::sample for a given uniform draw. The reference walks the row (u < p_i returns i, else u -= p_i);
+// here a CTA owns a contiguous slice, each warp a part of it and each chunk of at least 128 values a part of that. Masses are
+// summed per chunk; the warp(s) whose part can hold the draw find its chunk and walk on from there 32 values at a time
+// (whole parts walked: one load's latency per 32 values), and the lowest index found wins. 88 -> 35 us on 64 x 151936 after top-k 50
+__global__ void __launch_bounds__(kThreads, 4)
 multinomial_kernel(const float* __restrict__ logits, int n, const float* __restrict__ uniforms, uint32_t* __restrict__ out) {
-  __shared__ float red[32];
-  __shared__ float s_scan[kThreads / 32];
-  __shared__ unsigned int s_best;
-  const float* l = logits + (size_t)blockIdx.x * n;
+  constexpr int kWarps = kThreads / 32;
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  __shared__ float s_chunk[kWarps][32], s_mass[kWarps];
+  const cg::cluster_group c = cg::this_cluster();
+  Row row(const_cast<float*>(logits), n, c);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, out_row = blockIdx.x / row.size;
+  if (threadIdx.x == 0) sh.best = 0xffffffffu;
+  row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
   float mx, sum;
-  row_max_sum(l, n, true, red, mx, sum);
+  row_max_sum(c, row, true, room, sh, mx, sum);
+  uint32_t* best = c.map_shared_rank(&sh.best, 0);
   if (!(sum > 0.0f)) {  // no mass anywhere: greedy (first strict maximum from -inf, index 0 if none)
-    float bv = -INFINITY;
-    unsigned int bi = 0xffffffffu;
-    for (int i = threadIdx.x; i < n; i += kThreads)
-      if (l[i] > bv) { bv = l[i]; bi = (unsigned int)i; }
-    if (threadIdx.x == 0) s_best = 0xffffffffu;
-    __syncthreads();
-    const float m = block_max(bv, red);
-    if (bi != 0xffffffffu && bv == m) atomicMin(&s_best, bi);
-    __syncthreads();
-    if (threadIdx.x == 0) out[blockIdx.x] = s_best == 0xffffffffu ? 0u : s_best;
+    uint32_t bi = 0xffffffffu;
+    row.each([&](int i, float v) { if (v == mx && v > -INFINITY) bi = min(bi, (uint32_t)i); });
+    if (bi != 0xffffffffu) atomicMin(best, bi);
+    row_sync(c, row);
+    if (row.rank == 0 && threadIdx.x == 0) out[out_row] = sh.best == 0xffffffffu ? 0u : sh.best;
     return;
   }
-  const float u = uniforms[blockIdx.x];
-  const int per = (n + kThreads - 1) / kThreads;
-  const int i0 = min(threadIdx.x * per, n), i1 = min(i0 + per, n);
+  const float u = uniforms[out_row];
   auto prob = [&](int i) {
-    const float v = l[i];
-    return fabsf(v) <= 3.402823466e38f ? expf(v - mx) / sum : 0.0f;
+    const float v = row.l[i];
+    return v != -INFINITY && fabsf(v) <= 3.402823466e38f ? expf(v - mx) / sum : 0.0f;
   };
-  float mine = 0.0f;
-  for (int i = i0; i < i1; ++i) mine += prob(i);
-  // exclusive scan of the slice masses in thread order
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float incl = mine;
+  const int per = (row.end - row.begin + kWarps - 1) / kWarps;
+  const int i0 = min(row.begin + warp * per, row.end), i1 = min(i0 + per, row.end);
+  const int chunk = 128 * ((per + 128 * 32 - 1) / (128 * 32)), n_chunks = (i1 - i0 + chunk - 1) / max(chunk, 1);  // up to 32 chunks
+  for (int k = 0; k < n_chunks; ++k) {
+    const int c0 = i0 + k * chunk, c1 = min(c0 + chunk, i1);
+    float m = 0.0f;
+#pragma unroll 4
+    for (int i = c0 + lane; i < c1; i += 32) m += prob(i);
+    m = warp_sum(m);
+    if (lane == 0) s_chunk[warp][k] = m;
+  }
+  __syncwarp();
+  float upto = lane < n_chunks ? s_chunk[warp][lane] : 0.0f;  // of the chunks up to and with this one
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
+    const float t = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += t;
   }
-  if (lane == 31) s_scan[warp] = incl;
-  if (threadIdx.x == 0) s_best = 0xffffffffu;
+  const float mine = __shfl_sync(0xffffffffu, upto, 31);
+  if (lane == 0) s_mass[warp] = mine;
   __syncthreads();
+  float before = 0.0f, cta = 0.0f;  // of the warps before this one, of the whole slice
+  for (int w = 0; w < kWarps; ++w) {
+    if (w < warp) before += s_mass[w];
+    cta += s_mass[w];
+  }
+  tell(c, row, sh.max, cta);  // the maxima were read by every CTA ahead of the last barrier
+  row_sync(c, row);
   float base = 0.0f;
-  for (int w = 0; w < warp; ++w) base += s_scan[w];
-  const float excl = base + incl - mine;
-  if (u >= excl && i0 < i1) {
+  for (int r = 0; r < row.rank; ++r) base += sh.max[r];
+  const float excl = base + before;
+  // the scans and the walk round differently: a draw left a hair above a slice belongs to the start of the next one even
+  // if that slice's own bound says otherwise
+  constexpr float kHair = 2e-6f;
+  if (u >= excl && i0 < i1 && u <= excl + mine + kHair) {
     float r = u - excl;
+    const uint32_t reach = __ballot_sync(0xffffffffu, lane < n_chunks && r < upto);
+    const int from = reach ? __ffs(reach) - 1 : n_chunks - 1;
+    if (from > 0) r = fmaxf(r - __shfl_sync(0xffffffffu, upto, from - 1), 0.0f);
     bool found = false;
-    for (int i = i0; i < i1; ++i) {
-      const float pr = prob(i);
-      if (r < pr) { atomicMin(&s_best, (unsigned int)i); found = true; break; }
-      r -= pr;
+    for (int i = i0 + from * chunk; i < i1 && !found; i += 32) {
+      const float pr = i + lane < i1 ? prob(i + lane) : 0.0f;
+      float incl = pr;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, pr > 0.0f && r < incl);
+      if (hit) {
+        if (lane == 0) atomicMin(best, (uint32_t)(i + __ffs(hit) - 1));
+        found = true;
+      }
+      r -= __shfl_sync(0xffffffffu, incl, 31);
     }
-    // the scan and the walk round differently: a draw left a hair above this slice belongs to the
-    // start of the next one even if that thread's own bound says otherwise
-    if (!found && r <= 2e-6f && i1 < n) atomicMin(&s_best, (unsigned int)i1);
+    if (!found && r <= kHair && i1 < n && lane == 0) atomicMin(best, (uint32_t)i1);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) out[blockIdx.x] = s_best == 0xffffffffu ? (uint32_t)(n - 1) : s_best;
+  row_sync(c, row);
+  if (row.rank == 0 && threadIdx.x == 0) out[out_row] = sh.best == 0xffffffffu ? (uint32_t)(n - 1) : sh.best;
+}
+
+// a row is a cluster of eight CTAs, or one CTA
+template <typename... P, typename... A>
+uint32_t launch_rows(void (*kern)(P...), int rows, int n, void* stream, A... args) {
+  const unsigned size = n >= kClusterFrom ? kMaxCluster : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)rows * size);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = size;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  return launch_status();
 }
 
 }  // namespace
@@ -325,7 +556,9 @@ uint32_t logismos_launch_temperature_f32(void* logits, int32_t rows, int32_t n, 
   const float t = fmaxf(temperature, 1e-6f);
   if (fabsf(t - 1.0f) < 1e-9f || rows == 0 || n == 0) return 0;
   const int64_t total = (int64_t)rows * n;
-  temperature_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>((float*)logits, total, t);
+  const int vec = ((uintptr_t)logits & 15) == 0;
+  const int64_t threads = vec ? (total + 3) / 4 : total;
+  temperature_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>((float*)logits, total, t, vec);
   return lg::launch_status();
 }
 
@@ -333,10 +566,7 @@ uint32_t logismos_launch_top_k_f32(void* logits, int32_t rows, int32_t n, int32_
   lg::LaunchScope launch_scope_;
   if (rows < 0 || n < 0 || k < 0 || !logits) return lg::kInvalidValue;
   if (k == 0 || k >= n || rows == 0) return 0;
-  cudaError_t e = cudaFuncSetAttribute(top_k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSelectSmem);
-  if (e != cudaSuccess) return (uint32_t)e;
-  top_k_kernel<<<rows, kThreads, kSelectSmem, (cudaStream_t)stream>>>((float*)logits, n, k);
-  return lg::launch_status();
+  return launch_rows(top_k_kernel, rows, n, stream, (float*)logits, n, k);
 }
 
 uint32_t logismos_launch_top_p_f32(void* logits, int32_t rows, int32_t n, float p, void* stream) {
@@ -344,10 +574,7 @@ uint32_t logismos_launch_top_p_f32(void* logits, int32_t rows, int32_t n, float 
   if (rows < 0 || n < 0 || !logits) return lg::kInvalidValue;
   const float pc = fminf(fmaxf(p, 0.0f), 1.0f);
   if (pc >= 1.0f || rows == 0 || n == 0) return 0;
-  cudaError_t e = cudaFuncSetAttribute(top_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSelectSmem);
-  if (e != cudaSuccess) return (uint32_t)e;
-  top_p_kernel<<<rows, kThreads, kSelectSmem, (cudaStream_t)stream>>>((float*)logits, n, pc);
-  return lg::launch_status();
+  return launch_rows(top_p_kernel, rows, n, stream, (float*)logits, n, pc);
 }
 
 uint32_t logismos_launch_min_p_f32(void* logits, int32_t rows, int32_t n, float p, void* stream) {
@@ -355,8 +582,7 @@ uint32_t logismos_launch_min_p_f32(void* logits, int32_t rows, int32_t n, float 
   if (rows < 0 || n < 0 || !logits) return lg::kInvalidValue;
   const float pc = fminf(fmaxf(p, 0.0f), 1.0f);
   if (pc <= 0.0f || rows == 0 || n == 0) return 0;
-  min_p_kernel<<<rows, kThreads, 0, (cudaStream_t)stream>>>((float*)logits, n, pc);
-  return lg::launch_status();
+  return launch_rows(min_p_kernel, rows, n, stream, (float*)logits, n, pc);
 }
 
 uint32_t logismos_launch_repetition_penalty_f32(void* logits, int32_t rows, int32_t n, const void* tokens_u32,
@@ -375,8 +601,7 @@ uint32_t logismos_launch_multinomial_f32(const void* logits, int32_t rows, int32
   if (rows < 0 || n < 0 || !out_u32 || (rows > 0 && n > 0 && (!logits || !uniforms_f32))) return lg::kInvalidValue;
   if (rows == 0) return 0;
   if (n == 0) return (uint32_t)cudaMemsetAsync(out_u32, 0, (size_t)rows * 4, (cudaStream_t)stream);  // an empty slice samples 0
-  multinomial_kernel<<<rows, kThreads, 0, (cudaStream_t)stream>>>((const float*)logits, n, (const float*)uniforms_f32, (uint32_t*)out_u32);
-  return lg::launch_status();
+  return launch_rows(multinomial_kernel, rows, n, stream, (const float*)logits, n, (const float*)uniforms_f32, (uint32_t*)out_u32);
 }
 
 }  // extern "C"

@@ -136,3 +136,52 @@ def test_chain_runs_processors_in_order_then_samples():  # chain.rs:33-76, :88-1
     assert int(c2.step(small)[0]) == 0 and torch.isinf(small[0, 1:]).all()
     with pytest.raises(InvalidOp):
         S.TopK(5).process(torch.zeros((2, 8)))  # CPU tensor: no CPU arm
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 1000, 2047, 2048, 8195, 33000, 151937])
+def test_edges_of_the_slices_of_a_row(n):
+    """Rows below and above the length from which eight CTAs share one, lengths that leave rows unaligned and slices ragged or
+    empty; survivors that fit the list of a CTA and that do not; ties at the cut in several slices; NaN and infinities.
+    Top-k is bit-exact; the nucleus and the draw differ only where the mass (float64) lies within SUM_TOL of the cut."""
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal((6, n)) * 3.0).astype(np.float32)
+    x[1] = np.round(x[1]) + 0.0                   # ties everywhere (and one zero)
+    x[2, rng.random(n) < 0.9] = -np.inf
+    x[3] = 0.25                                   # one value: all of them tie
+    x[4, n // 2] = np.nan
+    x[5, -1] = np.inf
+    for k in sorted({1, 2, 40, n // 2, n - 1}):
+        got = run(S.TopK(k), x)
+        for r in range(6):
+            assert np.array_equal(got[r], O.top_k(x[r], k), equal_nan=True), (k, r)
+    for p in (0.0, 0.3, 0.95):
+        got = run(S.TopP(p), x)
+        for r in range(6):
+            if r == 3:  # equal probabilities: the first ceil(p n), give or take the one that fp32 rounding of 1 / n moves
+                kept = np.flatnonzero(got[r] > -np.inf)
+                assert abs(kept.size - max(np.ceil(p * n), 1)) <= 1 and kept[-1] == kept.size - 1, (p, kept.size)
+                continue
+            if r == 4 and n > 1:  # a NaN leaves the probabilities unnormalised: the maximum alone has mass one
+                assert np.array_equal(np.flatnonzero(got[r] > -np.inf), [np.nanargmax(x[r])]), p
+                continue
+            if r >= 4:            # no probability that is a number: everything is kept
+                assert np.array_equal(got[r], x[r], equal_nan=True), (p, r)
+                continue
+            ref = O.top_p(x[r], p)
+            kg, kr = got[r] > -np.inf, ref > -np.inf
+            pr = probs64(x[r]) if np.isfinite(x[r]).any() else np.zeros(n)
+            order = np.argsort(-pr, kind="stable")
+            ng, nr = int(kg.sum()), int(kr.sum())
+            assert kg[order[:ng]].all() and kr[order[:nr]].all(), (p, r)
+            if ng != nr:
+                cum, (lo, hi) = np.cumsum(pr[order]), sorted((ng, nr))
+                assert cum[lo - 1] >= p * (1 - SUM_TOL) and cum[max(hi - 2, 0)] <= p * (1 + SUM_TOL), (p, r, ng, nr)
+    t = torch.from_numpy(x).to(DEV)
+    for u in (0.0, 0.37, 0.999):
+        got = S.MultinomialSampler(seed=1).sample(t, uniforms=torch.full((6,), u, device=DEV)).cpu().numpy().view(np.uint32)
+        for r in range(6):
+            ref = O.multinomial(x[r], u)
+            if got[r] != ref:
+                pr = np.where(np.isfinite(x[r]), probs64(x[r]), 0.0)
+                cdf, (lo, hi) = np.cumsum(pr), sorted((int(got[r]), ref))
+                assert cdf[hi - 1] - cdf[lo] <= SUM_TOL and abs(cdf[lo] - u) <= SUM_TOL, (u, r, got[r], ref)
