@@ -61,6 +61,31 @@ inline void launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaS
   (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// The same for clusters of `cluster` blocks along x.
+template <typename... P, typename... A>
+inline void launch_cluster(void (*kern)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (dependent_launch()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // The same launch without the attribute: an ordinary stream-ordered launch, which starts only after
 // everything before it on the stream has completed. The model steps begin with one (the embedding
 // lookup), so a kernel of a step may read, ahead of its own dependency wait, anything that earlier

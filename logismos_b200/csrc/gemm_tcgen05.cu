@@ -2,20 +2,23 @@
 // (crates/kernels/src/cpu_f32/mod.rs:271-345) for the encoder / prefill GEMMs, which are the
 // only dense contractions on the path.
 //
-// Design (one persistent CTA per SM, 192 threads):
+// Design (one persistent CTA per SM, 320 threads):
 //   warp 0      TMA producer: cp.async.bulk.tensor 2-D tiles of A [128 x 64] and W [BN x 64]
 //               (bf16, 128-byte swizzle) into a ring of shared-memory stages
 //   warp 1      allocates TMEM and issues tcgen05.mma (cta_group::1, kind::f16, M=128, N=BN,
 //               K=16; four per 64-wide stage) with fp32 accumulators in TMEM; two accumulator
 //               buffers so the epilogue of tile i overlaps the main loop of tile i+1
-//   warps 2..5  epilogue: tcgen05.ld 32 lanes x 32 columns per warp step; bf16 outputs (bias,
-//               SwiGLU fused in registers) go out as 64-byte-per-thread vector stores; the fp32
+//   warps 2..9  epilogue, two warps per quarter of the tensor memory's lanes: tcgen05.ld 32 lanes x 32 columns per
+//               warp step; bf16 outputs leave through staging slabs as TMA stores, SwiGLU (fused in registers) as
+//               64-byte-per-thread vector stores; the fp32
 //               residual update x += acc is staged as 32 x 32 slabs in shared memory (128-byte
 //               swizzle) and applied by a TMA bulk tensor reduce-add, so x is never read into the SM
 // Synchronisation is by mbarriers only: full/empty per stage (TMA complete_tx, tcgen05.commit)
 // and full/empty per accumulator buffer. Every wait is bounded; on expiry the kernel raises an
 // error word, lets outstanding copies land, frees its TMEM and returns.
-// No cluster launch and no multicast is used: each CTA fetches its own tiles.
+// PAIR: a cluster of two CTAs computes tiles of 256 x 256 (cta_group::2): each fetches its 128 rows of A and half of
+// W's, so an SM reads 32 KB per k block instead of 48, and six stages fit; one thread of the first CTA issues the MMAs of both, each
+// CTA drains its own 128 rows. No multicast is used: each CTA fetches its own tiles.
 #include <cuda.h>
 
 #include <algorithm>
@@ -32,20 +35,21 @@ using namespace lg::tc;
 constexpr int BM = 128;
 constexpr int BK = 64;            // 64 bf16 = 128 B = one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int kThreads = 192;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 64 + 32 * kEpiWarps;
 
-template <int BN>
+// PAIR: a tile of 256 rows by a cluster of two CTAs, each with its 128 rows of A and half of W's
+template <int BN, bool PAIR = false>
 struct Cfg {
+  static constexpr int kRowsB = PAIR ? BN / 2 : BN;
   static constexpr int kStageA = BM * BK * 2;
-  static constexpr int kStageB = BN * BK * 2;
+  static constexpr int kStageB = kRowsB * BK * 2;
   static constexpr int kStage = kStageA + kStageB;
-  static constexpr int kStages = (192 * 1024) / kStage;  // 256->4, 192->4, 128->6
+  static constexpr int kStages = (192 * 1024) / kStage;  // 256->4, 192->4, 128->6; pairs 256->6, 192->6, 128->8
   static constexpr int kTmemCols = (2 * BN <= 256) ? 256 : 512;
-  static constexpr int kEpiBytes = 4 * 2 * 4096;  // 4 epilogue warps x 2 staging slabs of 32 rows x 128 B
+  static constexpr int kEpiBytes = kEpiWarps * 4096;  // a staging slab of 32 rows x 128 B per epilogue warp
   static constexpr size_t kSmem = (size_t)kStages * kStage + kEpiBytes + 1024 /*align*/ + 256 /*barriers*/;
 };
-
-LG_DEVINL float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 
 // eight bias values (the same for every lane); vec: the pointer is 16-byte aligned
 LG_DEVINL void load_bias8(const float* __restrict__ bias, bool vec, float (&b)[8]) {
@@ -99,13 +103,24 @@ struct RowTiles {
   int direct;          // 0: no group reads map_out
 };
 
-template <int BN, int EPI, bool EXPERTS = false>
+// Order of the output tiles: groups of `group` row tiles, in a group column tile by column tile. What runs at one time then
+// shares row and column tiles, and the larger operand is read from HBM once: 20384 x 1536 over k = 8960 (A alone is three
+// times L2) takes 523 us with all row tiles in one group, 402 with 16 of 128 rows or 4 of 256, 405 with 2 of 256.
+LG_DEVINL void tile_at(int t, int m_tiles, int n_tiles, int group, int& m_blk, int& n_blk) {
+  const int per = group * n_tiles, g = t / per, r = t - g * per;
+  const int rows = min(group, m_tiles - g * group);
+  n_blk = r / rows;
+  m_blk = g * group + r - n_blk * rows;
+}
+
+template <int BN, int EPI, bool EXPERTS = false, bool PAIR = false>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                         const __grid_constant__ CUtensorMap map_out, const float* __restrict__ bias,
-                        void* __restrict__ out, int M, int N, int K, int ldc, int splits, int w_static,
+                        void* __restrict__ out, int M, int N, int K, int ldc, int splits, int group, int w_static,
                         EpiParams ep, const lg_linear_groups_t groups, const RowTiles row_tiles, int* __restrict__ status) {
-  using C = Cfg<BN>;
+  using C = Cfg<BN, PAIR>;
+  constexpr int kTileM = PAIR ? 2 * BM : BM;
   lg::pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: required by the 128-byte swizzle atoms the descriptors assume
@@ -123,7 +138,9 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (EXPERTS) lg::pdl_wait();  // the tile list is the work of a kernel of this step
-  const int m_tiles = EXPERTS ? *row_tiles.n_tiles : (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
+  const int rank = PAIR ? (int)cluster_rank() : 0;  // 0 issues the MMAs of a pair
+  const int first_tile = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, tile_step = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+  const int m_tiles = EXPERTS ? *row_tiles.n_tiles : (M + kTileM - 1) / kTileM, n_tiles = (N + BN - 1) / BN;
   // a work item is (k slice, output tile); slices of k exist only for the accumulating epilogue, whose
   // reduce-add makes them meet in the output
   const int out_tiles = m_tiles * n_tiles;
@@ -133,7 +150,7 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(tfull_bar(b), 1); mbar_init(tempty_bar(b), 4); }
+    for (int b = 0; b < 2; ++b) { mbar_init(tfull_bar(b), 1); mbar_init(tempty_bar(b), (PAIR ? 2 : 1) * kEpiWarps); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -142,22 +159,36 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   // this CTA's first tile are requested before the dependency wait (they land while the preceding
   // kernel drains); each stage's barrier already expects the bytes of both halves
   int pre_w = 0;
-  if (w_static && threadIdx.x == 0 && (int)blockIdx.x < total_tiles) {
-    const int ot = (int)blockIdx.x % out_tiles, sp = (int)blockIdx.x / out_tiles;
-    const int n_blk = ot / m_tiles;
+  if (PAIR) cluster_sync();  // the barriers of both CTAs are there
+  // a stage of a pair is complete when the bytes of both CTAs have arrived at the first one's barrier
+  auto expect_stage = [&](int s) { if (rank == 0) mbar_expect_tx(full_bar(s), (uint32_t)C::kStage * (PAIR ? 2u : 1u)); };
+  auto load = [&](uint32_t dst, const CUtensorMap* map, int s, int x, int y) {
+    if (PAIR) tma_load_2d_pair(dst, map, peer_smem(full_bar(s), 0), x, y);
+    else tma_load_2d(dst, map, full_bar(s), x, y);
+  };
+  if (w_static && threadIdx.x == 0 && first_tile < total_tiles) {
+    const int ot = first_tile % out_tiles, sp = first_tile / out_tiles;
+    int m_blk, n_blk;
+    tile_at(ot, m_tiles, n_tiles, group, m_blk, n_blk);
     const int kb0 = sp * kb_per, kb1 = min(all_kb, kb0 + kb_per);
     for (int kb = kb0; kb < kb1 && pre_w < C::kStages; ++kb, ++pre_w) {
-      mbar_expect_tx(full_bar(pre_w), (uint32_t)C::kStage);
-      tma_load_2d(smem_base + pre_w * C::kStage + C::kStageA, &map_w, full_bar(pre_w), kb * BK, n_blk * BN);
+      expect_stage(pre_w);
+      load(smem_base + pre_w * C::kStage + C::kStageA, &map_w, pre_w, kb * BK, n_blk * BN + rank * C::kRowsB);
     }
   }
   if (!EXPERTS) lg::pdl_wait();  // everything before this touched shared memory or read the static weights only
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32((const void*)tmem_slot)), "r"((uint32_t)C::kTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32((const void*)tmem_slot)), "r"((uint32_t)C::kTmemCols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32((const void*)tmem_slot)), "r"((uint32_t)C::kTmemCols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // both CTAs have their tensor memory
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -167,12 +198,13 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
         const int ot = tile % out_tiles, sp = tile / out_tiles;
-        const int m_blk = ot % m_tiles, n_blk = ot / m_tiles;
+        int m_blk, n_blk;
+        tile_at(ot, m_tiles, n_tiles, group, m_blk, n_blk);
         const int kb0 = sp * kb_per, kb1 = min(all_kb, kb0 + kb_per);
         // a tile lies in one group of columns; rows beyond M read the next copy's and are not stored
-        int a_row = m_blk * BM + (EPI == kEpiGroups ? group_of(groups, n_blk * BN) * M : 0), w_row = n_blk * BN;
+        int a_row = m_blk * kTileM + rank * BM + (EPI == kEpiGroups ? group_of(groups, n_blk * BN) * M : 0), w_row = n_blk * BN + rank * C::kRowsB;
         const CUtensorMap* a_map = &map_a;
         if (EXPERTS) {
           const int4 rt = row_tiles.tiles[m_blk];
@@ -184,24 +216,29 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
           const bool have_w = pre_w > 0;  // requested before the dependency wait (first stages of the first tile)
-          if (!have_w) mbar_expect_tx(full_bar(stage), (uint32_t)C::kStage);
+          if (!have_w) expect_stage(stage);
           const uint32_t sa = smem_base + stage * C::kStage;
-          tma_load_2d(sa, a_map, full_bar(stage), kb * BK, a_row);
-          if (!have_w) tma_load_2d(sa + C::kStageA, &map_w, full_bar(stage), kb * BK, w_row);
+          load(sa, a_map, stage, kb * BK, a_row);
+          if (!have_w) load(sa + C::kStageA, &map_w, stage, kb * BK, w_row);
           else --pre_w;
           if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
         }
       }
+      // the peer's commits to this CTA's barriers are behind it before the CTA may retire
+      for (int i = 0; PAIR && ok && i < C::kStages; ++i) {
+        ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag);
+        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+      }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc<BN>();
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = make_idesc<BN, kTileM>();
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+      for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++it) {
         const int buf = it & 1;
         const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
         if (!mbar_wait(tempty_bar(buf), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
@@ -217,72 +254,77 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // advancing 16 bf16 along K inside the swizzle row = +32 B = +2 in the encoded address
-            tc_mma_bf16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, ((kb - kb0) | k) ? 1u : 0u);
+            if (PAIR) tc_mma_bf16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, ((kb - kb0) | k) ? 1u : 0u);
+            else tc_mma_bf16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, ((kb - kb0) | k) ? 1u : 0u);
           }
-          tc_commit(empty_bar(stage));  // stage reusable once these MMAs have read it
+          // stage reusable once these MMAs have read it
+          if (PAIR) tc_commit_pair(empty_bar(stage));
+          else tc_commit(empty_bar(stage));
           if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) tc_commit(tfull_bar(buf));  // accumulator complete
+        if (ok) {  // accumulator complete
+          if (PAIR) tc_commit_pair(tfull_bar(buf));
+          else tc_commit(tfull_bar(buf));
+        }
       }
     }
   } else {
-    // ---------------- epilogue (warps 2..5) ----------------
-    const int q = warp & 3;  // TMEM lane quarter this warp may access
-    uint8_t* slabs = smem_gen + C::kStages * C::kStage + q * 2 * 4096;
-    const uint32_t slabs_a = epi_base + q * 2 * 4096;
-    int it = 0, n_store = 0;
+    // ---------------- epilogue (warps 2..9) ----------------
+    const int q = warp & 3;               // TMEM lane quarter this warp may access
+    const int c0 = ((warp - 2) >> 2) * 64;  // the two warps of a quarter take 64 columns in turn
+    uint8_t* slab = smem_gen + C::kStages * C::kStage + (warp - 2) * 4096;
+    const uint32_t slab_a = epi_base + (warp - 2) * 4096;
+    int it = 0;
     const bool bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
     bool ok = true;
-    // hands the slab just written to the TMA engine; the slab used two stores ago must have been read
-    auto slab_acquire = [&]() -> int {
-      const int b = n_store & 1;
-      if (lane == 0) bulk_wait_read<1>();
+    // hands the slab just written to the TMA engine, which must have read what was in it before
+    auto slab_acquire = [&]() {
+      if (lane == 0) bulk_wait_read<0>();
       __syncwarp();
-      return b;
     };
-    auto slab_release = [&](int b, int x, int y, bool in_range) {
+    auto slab_release = [&](int x, int y, bool in_range) {
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) {
         if (in_range) {
-          if (EPI == LG_EPI_RESID_F32) tma_reduce_add_2d(&map_out, slabs_a + b * 4096, x, y);
-          else tma_store_2d(&map_out, slabs_a + b * 4096, x, y);
+          if (EPI == LG_EPI_RESID_F32) tma_reduce_add_2d(&map_out, slab_a, x, y);
+          else tma_store_2d(&map_out, slab_a, x, y);
         }
         bulk_commit();
       }
-      ++n_store;
     };
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++it) {
       const int ot = tile % out_tiles;
-      const int m_blk = ot % m_tiles, n_blk = ot / m_tiles;
+      int m_blk, n_blk;
+      tile_at(ot, m_tiles, n_tiles, group, m_blk, n_blk);
       const bool first_slice = tile < out_tiles;  // the bias joins once
       const int buf = it & 1;
       const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
       if (!mbar_wait_warp(tfull_bar(buf), acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      const int4 rt = EXPERTS ? row_tiles.tiles[m_blk] : make_int4(0, m_blk * BM, M, 0);
+      const int4 rt = EXPERTS ? row_tiles.tiles[m_blk] : make_int4(0, m_blk * kTileM + rank * BM, M, 0);
       const int row0 = rt.y + q * 32;  // first output row of this warp's slab
       const int row = row0 + lane, row_end = rt.z;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
       if (EPI == LG_EPI_RESID_F32) {
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = c0; c < BN; c += (c & 32) ? 96 : 32) {
           uint32_t r[32];
           tc_ld32(t_row + c, r);
           tc_wait_ld();
           const int ncol = n_blk * BN + c;
-          const int b = slab_acquire();
+          slab_acquire();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             float a0 = __uint_as_float(r[4 * j]), a1 = __uint_as_float(r[4 * j + 1]);
             float a2 = __uint_as_float(r[4 * j + 2]), a3 = __uint_as_float(r[4 * j + 3]);
             if (bias && first_slice && ncol + 4 * j < N) { a0 += bias[ncol + 4 * j]; a1 += bias[ncol + 4 * j + 1]; a2 += bias[ncol + 4 * j + 2]; a3 += bias[ncol + 4 * j + 3]; }
-            slab_write(slabs + b * 4096, lane, j, make_uint4(__float_as_uint(a0), __float_as_uint(a1), __float_as_uint(a2), __float_as_uint(a3)));
+            slab_write(slab, lane, j, make_uint4(__float_as_uint(a0), __float_as_uint(a1), __float_as_uint(a2), __float_as_uint(a3)));
           }
-          slab_release(b, ncol, row0, ncol < N && row0 < M);
+          slab_release(ncol, row0, ncol < N && row0 < M);
         }
       } else if (!EXPERTS && (EPI == LG_EPI_BF16 || EPI == LG_EPI_RELU2 || EPI == kEpiGroups)) {  // 64 columns at a time through the staging slabs
         const int n_out = EPI == kEpiGroups ? groups.n_main : N;
-        for (int c = 0; c < BN; c += 64) {
+        for (int c = c0; c < BN; c += 128) {
           const int ncol = n_blk * BN + c;
           if (ncol >= N) break;
           uint32_t ra[32], rb[32];
@@ -296,7 +338,7 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             }
             continue;
           }
-          const int b = slab_acquire();
+          slab_acquire();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int col = ncol + 8 * j;
@@ -312,12 +354,12 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
               if (silu) { x = lg::silu_fast(x); y = lg::silu_fast(y); }
               w[i] = pack_bf16x2(x, y);
             }
-            slab_write(slabs + b * 4096, lane, j, make_uint4(w[0], w[1], w[2], w[3]));
+            slab_write(slab, lane, j, make_uint4(w[0], w[1], w[2], w[3]));
           }
-          slab_release(b, ncol, row0, row0 < M);
+          slab_release(ncol, row0, row0 < M);
         }
       } else if (EPI == LG_EPI_BF16) {  // a group's rows may end inside a tile
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = c0; c < BN; c += (c & 32) ? 96 : 32) {
           uint32_t r[32];
           tc_ld32(t_row + c, r);
           tc_wait_ld();
@@ -336,13 +378,13 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
           }
         }
       } else if (EPI == LG_EPI_F32 && (ldc & 3) == 0) {  // whole 128-byte rows through the staging slabs
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = c0; c < BN; c += (c & 32) ? 96 : 32) {
           uint32_t r[32];
           tc_ld32(t_row + c, r);
           tc_wait_ld();
           const int ncol = n_blk * BN + c;
           if (ncol >= N) break;
-          const int b = slab_acquire();
+          slab_acquire();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             float v[4];
@@ -352,12 +394,12 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
               if (bias && ncol + 4 * j + i < N) v[i] += bias[ncol + 4 * j + i];
               if (ep.p0 > 0.0f) v[i] = ep.p0 * tanhf(v[i] / ep.p0);
             }
-            slab_write(slabs + b * 4096, lane, j, make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])));
+            slab_write(slab, lane, j, make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])));
           }
-          slab_release(b, ncol, row0, row0 < M);
+          slab_release(ncol, row0, row0 < M);
         }
       } else if (EPI == LG_EPI_F32) {
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = c0; c < BN; c += (c & 32) ? 96 : 32) {
           uint32_t r[32];
           tc_ld32(t_row + c, r);
           tc_wait_ld();
@@ -380,7 +422,7 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         }
       } else {  // LG_EPI_SWIGLU, LG_EPI_GLU_CLAMP
         // W rows interleave 32 gate rows with the 32 matching up rows
-        for (int c = 0; c < BN; c += 64) {
+        for (int c = c0; c < BN; c += 128) {
           uint32_t g[32], u[32];
           tc_ld32(t_row + c, g);
           tc_ld32(t_row + c + 32, u);
@@ -403,7 +445,7 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 const float g0 = __uint_as_float(g[e]) + bg[2 * i], g1 = __uint_as_float(g[e + 1]) + bg[2 * i + 1];
                 const float u0 = __uint_as_float(u[e]) + bu[2 * i], u1 = __uint_as_float(u[e + 1]) + bu[2 * i + 1];
                 if (EPI == LG_EPI_GLU_CLAMP) w[i] = pack_bf16x2(lg::glu_clamp(g0, u0, ep.p0, ep.p1, ep.p2), lg::glu_clamp(g1, u1, ep.p0, ep.p1, ep.p2));
-                else w[i] = pack_bf16x2(silu_f(g0) * u0, silu_f(g1) * u1);
+                else w[i] = pack_bf16x2(lg::silu_fast(g0) * u0, lg::silu_fast(g1) * u1);
               }
               *reinterpret_cast<uint4*>(dst + j * 8) = make_uint4(w[0], w[1], w[2], w[3]);
             }
@@ -412,7 +454,10 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(tempty_bar(buf));
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(peer_smem(tempty_bar(buf), 0));
+        else mbar_arrive(tempty_bar(buf));
+      }
     }
     if (lane == 0) bulk_wait_all();  // every slab has left shared memory and landed before the CTA retires
   }
@@ -427,9 +472,11 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // neither CTA of a pair leaves while the other may use its barriers or tensor memory
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)C::kTmemCols) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)C::kTmemCols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)C::kTmemCols) : "memory");
   }
 }
 
@@ -453,13 +500,22 @@ __global__ void linear_t_naive_kernel(const __nv_bfloat16* __restrict__ a, const
 
 // ---- host side ------------------------------------------------------------------------------------
 
-template <int BN, int EPI>
+// few output tiles and a long reduction (the output projections of a small step): the accumulating
+// epilogue lets slices of k run on otherwise idle SMs; every slice gets at least four k blocks
+inline int k_splits(int64_t tiles, int workers, int all_kb) {
+  if (lg::deterministic() || tiles * 2 > workers || all_kb < 8) return 1;
+  const int want = (int)(workers / tiles);
+  const int kb_per = std::max(4, (all_kb + want - 1) / want);
+  return (all_kb + kb_per - 1) / kb_per;
+}
+
+template <int BN, int EPI, bool PAIR = false>
 uint32_t launch_cfg(const void* a, const void* w, const float* bias, void* out, int m, int n, int k, int lda,
                     int ldc, int w_static, EpiParams ep, int* status, cudaStream_t stream, const lg_linear_groups_t& groups = {}) {
   CUtensorMap ma, mw, mo;
   const int copies = EPI == kEpiGroups ? groups.n_groups : 1;
   if (!make_map(&ma, a, (uint64_t)m * copies, (uint64_t)k, (uint64_t)lda, BM)) return lg::kInvalidValue;
-  if (!make_map(&mw, w, (uint64_t)n, (uint64_t)k, (uint64_t)k, BN)) return lg::kInvalidValue;
+  if (!make_map(&mw, w, (uint64_t)n, (uint64_t)k, (uint64_t)k, Cfg<BN, PAIR>::kRowsB)) return lg::kInvalidValue;
   if (EPI == LG_EPI_RESID_F32 || (EPI == LG_EPI_F32 && ldc % 4 == 0)) {  // fp32 [m, n] in 32 x 32 boxes
     if (!make_map(&mo, out, (uint64_t)m, (uint64_t)n, (uint64_t)ldc, 32, true)) return lg::kInvalidValue;
   } else if (EPI == LG_EPI_BF16 || EPI == LG_EPI_RELU2 || (EPI == kEpiGroups && groups.n_main > 0)) {  // bf16 in 32 x 64 boxes
@@ -467,52 +523,57 @@ uint32_t launch_cfg(const void* a, const void* w, const float* bias, void* out, 
   } else {
     mo = ma;  // unused by the direct-store epilogues
   }
-  auto kern = linear_t_tcgen05_kernel<BN, EPI>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<BN>::kSmem);
+  auto kern = linear_t_tcgen05_kernel<BN, EPI, false, PAIR>;
+  using C = Cfg<BN, PAIR>;
+  constexpr int kTileM = PAIR ? 2 * BM : BM;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
   if (e != cudaSuccess) return (uint32_t)e;
-  const int tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
-  // few output tiles and a long reduction (the output projections of a small step): the accumulating
-  // epilogue lets slices of k run on otherwise idle SMs; every slice gets at least four k blocks
-  int splits = 1;
-  if (EPI == LG_EPI_RESID_F32 && !lg::deterministic()) {
-    const int all_kb = k / BK;
-    if (tiles * 2 <= sm_count() && all_kb >= 8) {
-      const int want = sm_count() / tiles;
-      int kb_per = (all_kb + want - 1) / want;
-      if (kb_per < 4) kb_per = 4;
-      splits = (all_kb + kb_per - 1) / kb_per;
-    }
-  }
-  const int items = tiles * splits;
-  const int grid = items < sm_count() ? items : sm_count();
-  lg::launch(kern, dim3(grid), dim3(kThreads), Cfg<BN>::kSmem, stream, ma, mw, mo, bias, out, m, n, k, ldc, splits, w_static, ep, groups, RowTiles{}, status);
+  const int workers = PAIR ? sm_count() / 2 : sm_count();
+  const int tiles = ((m + kTileM - 1) / kTileM) * ((n + BN - 1) / BN);
+  const int splits = EPI == LG_EPI_RESID_F32 ? k_splits(tiles, workers, k / BK) : 1;
+  const int items = tiles * splits, group = PAIR ? 4 : 16;
+  const int grid = (items < workers ? items : workers) * (PAIR ? 2 : 1);
+  lg::launch_cluster(kern, PAIR ? 2 : 1, dim3(grid), dim3(kThreads), C::kSmem, stream, ma, mw, mo, bias, out, m, n, k, ldc, splits, group, w_static, ep,
+                     groups, RowTiles{}, status);
   return lg::launch_status();
 }
 
 template <int EPI>
 uint32_t launch_epi(const void* a, const void* w, const float* bias, void* out, int m, int n, int k, int lda,
                     int ldc, int w_static, EpiParams ep, int* status, cudaStream_t stream, const lg_linear_groups_t& groups = {}) {
-  // tile width by wave quantisation: time ~ waves(BN) * BN; ties go to the wider tile
-  const int sms = sm_count();
-  const int mt = (m + BM - 1) / BM;
-  int best_bn = 256;
-  long best_cost = -1;
-  const int cands[3] = {256, 192, 128};
-  for (int i = 0; i < 3; ++i) {
-    const int bn = cands[i];
+  // The tile by an estimate of its time: waves of tiles x k blocks x the time of a k block of that tile, in hundredths of
+  // a 128 x 256 one's (0.45 us when the chip is full: it then runs at the power limit). Measured at 700 to 2929 rows, 17920
+  // and 1536 columns: 192 columns 0.85 to 0.96, 128 columns 0.75 to 0.82 (their operands are read more often per product), 256
+  // x 256 by a pair of CTAs 0.84 to 0.93, and a pair starts 1.6 us later. 20384 x 1536 over k = 8960: 714 us as 128 columns (the
+  // choice by waves x columns), 446 as 256, 399 by pairs; 20384 x 17920 with SwiGLU 1008 -> 906; 2112 x 1536 over 8960 60 -> 54.
+  struct Tile { int bn, pair, kb_cost; };
+  const Tile tiles[4] = {{256, 0, 100}, {192, 0, 92}, {128, 0, 82}, {256, 1, 86}};
+  constexpr int64_t kPairStart = 350;
+  const int sms = sm_count(), all_kb = k / BK;
+  const bool one_row_tile = m <= BM;  // the time is that of the weights' way to the SMs: as many SMs as possible, few slices of k
+  Tile best = tiles[0];
+  int64_t best_cost = -1;
+  for (const Tile& t : tiles) {
+    if (t.pair && one_row_tile) continue;
     if (EPI == kEpiGroups) {  // a tile must not straddle two groups
-      bool fits = groups.n_main % bn == 0 || groups.n_main == n;
-      for (int g = 0; g + 1 < groups.n_groups; ++g) fits = fits && groups.end[g] % bn == 0;
+      bool fits = groups.n_main % t.bn == 0 || groups.n_main == n;
+      for (int g = 0; g + 1 < groups.n_groups; ++g) fits = fits && groups.end[g] % t.bn == 0;
       if (!fits) continue;
     }
-    const long tiles = (long)mt * ((n + bn - 1) / bn);
-    const long waves = (tiles + sms - 1) / sms;
-    long cost = waves * bn;
-    if (EPI == kEpiGroups && bn == 128) cost += cost / 6;  // the narrow tile runs at about six sevenths of the wide one's rate
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best_bn = bn; }
+    const int rows = t.pair ? 2 * BM : BM, workers = t.pair ? sms / 2 : sms;
+    const int64_t n_tiles = (int64_t)((m + rows - 1) / rows) * ((n + t.bn - 1) / t.bn);
+    int64_t cost;
+    if (one_row_tile) {
+      cost = (n_tiles + sms - 1) / sms * t.bn;
+    } else {
+      const int splits = EPI == LG_EPI_RESID_F32 ? k_splits(n_tiles, workers, all_kb) : 1;
+      cost = (n_tiles * splits + workers - 1) / workers * ((all_kb + splits - 1) / splits) * t.kb_cost + (t.pair ? kPairStart : 0);
+    }
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = t; }
   }
-  if (best_bn == 256) return launch_cfg<256, EPI>(a, w, bias, out, m, n, k, lda, ldc, w_static, ep, status, stream, groups);
-  if (best_bn == 192) return launch_cfg<192, EPI>(a, w, bias, out, m, n, k, lda, ldc, w_static, ep, status, stream, groups);
+  if (best.pair) return launch_cfg<256, EPI, true>(a, w, bias, out, m, n, k, lda, ldc, w_static, ep, status, stream, groups);
+  if (best.bn == 256) return launch_cfg<256, EPI>(a, w, bias, out, m, n, k, lda, ldc, w_static, ep, status, stream, groups);
+  if (best.bn == 192) return launch_cfg<192, EPI>(a, w, bias, out, m, n, k, lda, ldc, w_static, ep, status, stream, groups);
   return launch_cfg<128, EPI>(a, w, bias, out, m, n, k, lda, ldc, w_static, ep, status, stream, groups);
 }
 
@@ -540,7 +601,7 @@ uint32_t launch_experts(const ExpertRows& x, const void* w, void* out, int n, in
   if (e != cudaSuccess) return (uint32_t)e;
   const int64_t items = (int64_t)x.max_tiles * ((n + BN - 1) / BN);
   const int grid = items < sm_count() ? (int)items : sm_count();
-  lg::launch(kern, dim3(grid), dim3(kThreads), Cfg<BN>::kSmem, stream, ma, mw, md, (const float*)nullptr, out, x.a_rows, n, k, ldc, 1, 0, ep, lg_linear_groups_t{},
+  lg::launch(kern, dim3(grid), dim3(kThreads), Cfg<BN>::kSmem, stream, ma, mw, md, (const float*)nullptr, out, x.a_rows, n, k, ldc, 1, x.max_tiles, 0, ep, lg_linear_groups_t{},
              x.tiles, status);
   return lg::launch_status();
 }

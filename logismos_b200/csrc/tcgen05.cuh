@@ -124,6 +124,47 @@ LG_DEVINL void tc_mma_bf16(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, ui
       : "memory");
 }
 
+// ---- a pair of CTAs (cluster of two) on one tile of 256 rows: cta_group::2 ------------------------
+
+// the address of the same shared-memory location in CTA `rank` of the cluster
+LG_DEVINL uint32_t peer_smem(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+LG_DEVINL uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+LG_DEVINL void cluster_sync() {
+  asm volatile("barrier.cluster.arrive;\nbarrier.cluster.wait;\n" ::: "memory");
+}
+// a tile to this CTA's shared memory whose bytes a barrier of either CTA of the pair counts
+LG_DEVINL void tma_load_2d_pair(uint32_t smem_dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+      ::"r"(smem_dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y)
+      : "memory");
+}
+// arrives at the same barrier of both CTAs once the MMAs issued so far are done
+LG_DEVINL void tc_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar), "h"((uint16_t)3)
+               : "memory");
+}
+LG_DEVINL void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_bar) : "memory");
+}
+// rows 0..127 of A, the first half of B's rows and of D come from and go to the CTA that issues, the rest its peer's
+LG_DEVINL void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 LG_DEVINL void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -183,10 +224,10 @@ LG_DEVINL uint64_t make_smem_desc(uint32_t smem_addr) {
   return d;
 }
 
-// Instruction descriptor for kind::f16: D fp32, A and B bf16, both K-major, M=128, N=BN.
-template <int BN>
+// Instruction descriptor for kind::f16: D fp32, A and B bf16, both K-major, M=128 (256 for a pair of CTAs), N=BN.
+template <int BN, int M = 128>
 __host__ __device__ constexpr uint32_t make_idesc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // ---- host side ------------------------------------------------------------------------------------

@@ -97,3 +97,33 @@ def test_shape_guards_reject_before_launch():
         ops.linear_t(a, w)
     with pytest.raises(ops.InvalidOp):
         ops.linear_t(a.cpu(), w)
+
+
+# tiles of 256 rows by a pair of CTAs: rows that leave the second CTA's half of the last tile empty, ragged or whole, a ragged
+# last column tile, several groups of row tiles, k slices, every epilogue. Against fp32 products of the same bf16 values:
+# one bf16 rounding (2^-9 of the value), fp32 sums in another order (1e-4 of the largest)
+@pytest.mark.parametrize("m,n,k,kind", [(4161, 4112, 1024, "bf16"), (4224, 4096, 1024, "swiglu"), (2177, 1536, 8960, "resid"), (1089, 1536, 8960, "resid"), (4300, 4112, 1024, "f32"),
+                                        (4097, 4096, 1024, "f32")])
+def test_row_tiles_of_a_pair_of_ctas(m, n, k, kind):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(m + n)
+    a = torch.randn((m, k), generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn((n, k), generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    ref = a.float() @ w.float().T
+    if kind == "swiglu":
+        z = ref.reshape(m, n // 64, 2, 32)
+        ref = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(m, n // 2)
+        got = ops.linear_t(a, w, swiglu=True)
+    elif kind == "resid":
+        x = torch.randn((m, n), generator=g, device=DEV)
+        ref = x + ref
+        got = x.clone()
+        ops.linear_t(a, w, residual=got)
+    elif kind == "bf16":
+        bias = torch.randn(n, generator=g, device=DEV)
+        ref = ref + bias
+        got = ops.linear_t(a, w, bias)
+    else:
+        got = ops.linear_act(a, w, epilogue=ops.EPI_F32)
+    rounding = 0.0 if kind in ("resid", "f32") else 2 ** -8
+    assert ((got.float() - ref).abs() <= rounding * ref.abs() + 1e-4 * ref.abs().max()).all()
