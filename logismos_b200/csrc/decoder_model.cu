@@ -51,6 +51,7 @@ struct Decoder {
   // workspace
   Buf x, h, qkv, attn, qdec, gu, act, wscratch, accws, last, last_bf16, logits, tokens, status;
   Buf ids, pos, slots, cu_prefill, last_idx, dec_ctx, dec_tables, dec_chunks, dec_scratch, attn_ws, pre_kv;
+  HostRows host_rows;
   StepBatch batch;  // the last step (kept for replay and diagnostics)
   cudaStream_t stream = nullptr;
   std::mutex mu;
@@ -274,6 +275,7 @@ void lg_decoder_destroy(void* model) {
     for (Buf* b : lb) b->release();
   }
   m->batch.release();
+  m->host_rows.release();
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
 }
@@ -351,14 +353,13 @@ uint32_t lg_decoder_last_hidden(void* model, int32_t n_seqs, float* host_out) {
 
 uint32_t lg_decoder_last_logits(void* model, int32_t n_seqs, float* host_out) {
   Decoder* m = static_cast<Decoder*>(model);
+  std::lock_guard<std::mutex> lock(m->mu);
   if (n_seqs != m->n_seqs) { set_error("lg_decoder_last_logits: n_seqs differs from the last step"); return LG_EMB_COMPUTE; }
   cudaSetDevice(m->device);
   const size_t V = m->cfg.vocab;
   LG_TRY(cudaDeviceSynchronize(), "device synchronize");
   if (m->logits_f32) {
-    std::vector<float> tmp((size_t)n_seqs * V);
-    LG_TRY(cudaMemcpy(tmp.data(), m->logits.p, tmp.size() * 4, cudaMemcpyDeviceToHost), "D2H logits");
-    for (int k = 0; k < n_seqs; ++k) std::memcpy(host_out + (size_t)m->batch.order[k] * V, tmp.data() + (size_t)k * V, V * 4);
+    LG_TRY(m->host_rows.copy(m->logits.p, n_seqs, V, m->batch.order.data(), host_out, m->stream), "D2H logits");
     return LG_EMB_OK;
   }
   std::vector<uint16_t> tmp((size_t)n_seqs * V);

@@ -63,6 +63,7 @@ struct Hybrid {
   Buf gdn_scratch;  // per (chunk, head) intermediates of the chunk-parallel recurrence (two-launch form)
   Buf gdn_pairs;    // arrival counters of the fused decode kernel's CTA pairs, all zero between launches
   Buf ids, pos, slots, cu_all, cu_prefill, last_idx, dec_ctx, dec_tables, dec_chunks, dec_scratch, attn_ws, state_slots, fresh, pre_kv;
+  HostRows host_rows;
   StepBatch batch;  // the last step (kept for replay and diagnostics)
   cudaStream_t stream = nullptr;
   std::mutex mu;
@@ -384,6 +385,7 @@ void lg_hybrid_destroy(void* model) {
     for (Buf* b : lb) b->release();
   }
   m->batch.release();
+  m->host_rows.release();
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
 }
@@ -477,13 +479,12 @@ uint32_t lg_hybrid_last_hidden(void* model, int32_t n_seqs, float* host_out) {
 uint32_t lg_hybrid_last_logits(void* model, int32_t n_seqs, float* host_out) {
   Hybrid* m = static_cast<Hybrid*>(model);
   if (!m->logits_f32) return read_rows_bf16(m, m->logits, n_seqs, (size_t)m->cfg.vocab, host_out, "lg_hybrid_last_logits");
+  std::lock_guard<std::mutex> lock(m->mu);
   if (n_seqs != m->n_seqs) { set_error("lg_hybrid_last_logits: n_seqs differs from the last step"); return LG_EMB_COMPUTE; }
   cudaSetDevice(m->device);
   const size_t V = (size_t)m->cfg.vocab;
-  std::vector<float> tmp((size_t)n_seqs * V);
   LG_TRY(cudaDeviceSynchronize(), "device synchronize");
-  LG_TRY(cudaMemcpy(tmp.data(), m->logits.p, tmp.size() * 4, cudaMemcpyDeviceToHost), "D2H logits");
-  for (int k = 0; k < n_seqs; ++k) std::memcpy(host_out + (size_t)m->batch.order[k] * V, tmp.data() + (size_t)k * V, V * 4);
+  LG_TRY(m->host_rows.copy(m->logits.p, n_seqs, V, m->batch.order.data(), host_out, m->stream), "D2H logits");
   return LG_EMB_OK;
 }
 

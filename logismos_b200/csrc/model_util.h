@@ -2,10 +2,12 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "logismos_kernels.h"
@@ -28,6 +30,86 @@ struct Buf {
   bool alloc(size_t n) { return cudaMalloc(&p, n ? n : 1) == cudaSuccess; }
   bool upload(const void* src, size_t n) { return alloc(n) && cudaMemcpy(p, src, n, cudaMemcpyHostToDevice) == cudaSuccess; }
   void release() { if (p) cudaFree(p); p = nullptr; }
+};
+
+// Rows of fp32 from the device to pageable host memory, each to a place of its own. A copy into pageable memory goes through
+// the driver's staging at a few GB/s, and a temporary of the same size costs its page faults besides: 64 rows of 32768
+// took 2.0 ms that way. Here the rows land in a pinned buffer of at most kCap bytes, part by part, and up to four threads
+// move a part on while the next ones arrive: 0.5 ms, most of it the page faults of the destination.
+struct HostRows {
+  static constexpr size_t kCap = (size_t)16 << 20, kParts = 4, kAlone = (size_t)1 << 20;
+  uint8_t* pinned = nullptr;
+  size_t capacity = 0;
+  cudaEvent_t landed[kParts] = {};
+
+  void release() {
+    if (pinned) cudaFreeHost(pinned);
+    pinned = nullptr;
+    capacity = 0;
+    for (cudaEvent_t& e : landed) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
+  }
+
+  // row k of dev [rows][width] to host_out + order[k] * width; nothing on the device writes the rows meanwhile
+  cudaError_t copy(const void* dev, int rows, size_t width, const int* order, float* host_out, cudaStream_t s) {
+    const size_t row = width * 4, want = std::max(row, std::min(kCap, row * (size_t)rows));
+    if (rows <= 0 || row == 0) return cudaSuccess;
+    if (capacity < want) {
+      release();
+      if (cudaMallocHost((void**)&pinned, want) != cudaSuccess) {
+        pinned = nullptr;
+        (void)cudaGetLastError();
+      } else {
+        capacity = want;
+      }
+    }
+    for (cudaEvent_t& e : landed)
+      if (pinned && !e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return cudaGetLastError();
+    if (!pinned) {  // no pinned memory to be had: straight to the destination
+      for (int k = 0; k < rows; ++k) {
+        const cudaError_t e = cudaMemcpy(host_out + (size_t)order[k] * width, (const uint8_t*)dev + (size_t)k * row, row, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return e;
+      }
+      return cudaSuccess;
+    }
+    const int room = (int)std::min<size_t>(capacity / row, (size_t)rows);
+    for (int r0 = 0; r0 < rows; r0 += room) {
+      const int n = std::min(room, rows - r0), parts = (size_t)n * row <= kAlone ? 1 : std::min<int>((int)kParts, n);
+      cudaError_t err[kParts] = {};
+      for (int i = 0; i < parts; ++i) {
+        const int a = n * i / parts, b = n * (i + 1) / parts;
+        cudaError_t e = cudaMemcpyAsync(pinned + (size_t)a * row, (const uint8_t*)dev + (size_t)(r0 + a) * row, (size_t)(b - a) * row, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaEventRecord(landed[i], s);
+        if (e != cudaSuccess) {
+          (void)cudaStreamSynchronize(s);  // nothing is on its way to the buffer when it is given up
+          return e;
+        }
+      }
+      auto part = [&](int i) {
+        err[i] = cudaEventSynchronize(landed[i]);
+        if (err[i] != cudaSuccess) return;
+        for (int k = n * i / parts; k < n * (i + 1) / parts; ++k) std::memcpy(host_out + (size_t)order[r0 + k] * width, pinned + (size_t)k * row, row);
+      };
+      std::thread helpers[kParts];
+      bool helped[kParts] = {};
+      for (int i = 1; i < parts; ++i) {
+        try {
+          helpers[i] = std::thread(part, i);
+          helped[i] = true;
+        } catch (...) {
+        }  // no thread to be had: this one does its part
+      }
+      for (int i = 0; i < parts; ++i)
+        if (!helped[i]) part(i);
+      for (int i = 1; i < parts; ++i)
+        if (helped[i]) helpers[i].join();
+      for (int i = 0; i < parts; ++i)
+        if (err[i] != cudaSuccess) return err[i];
+    }
+    return cudaSuccess;
+  }
 };
 
 // an int4 matrix on the device; `dense` is its optional bf16 expansion [n, k], made once at load for
