@@ -81,8 +81,22 @@ uint32_t run_device(Decoder* m, cudaStream_t s) {
   }
   LG_TRY(logismos_launch_embed_lookup_bf16(m->tok_embed.p, m->ids.p, m->x.p, T, H, c.vocab, s), "embed_lookup");
   m->launches += 1;
+  const bool few = m->n_pre == 0 && lg::int4_rows_fit(T, std::max(H, I)) && !c.kv_turbo3;
   for (int l = 0; l < c.n_layers; ++l) {
     DLayer& L = m->layers[l];
+    if (few) {
+      const lg::DecodeHeads heads{D, c.n_heads, c.n_kv_heads, c.max_pos, (const float*)m->cos.p, (const float*)m->sin.p, (const int*)m->pos.p, (const int64_t*)m->slots.p,
+                                  (int64_t)c.n_pool_blocks * kBlock, (__nv_bfloat16*)m->qdec.p, (__nv_bfloat16*)L.kpool.p, (__nv_bfloat16*)L.vpool.p, nullptr, 0, (int*)st};
+      LG_TRY(few_heads(m->x, L.norm1, c.rms_eps, L.wqkv, L.bqkv.p, heads, T, &m->launches, s), "norm, qkv, rope and cache store of few rows");
+      LG_TRY(logismos_launch_paged_attention_decode_bf16(m->qdec.p, L.kpool.p, L.vpool.p, nullptr, nullptr, m->dec_tables.p, m->dec_ctx.p, m->dec_chunks.p, m->attn.p,
+                                                         m->dec_scratch.p, st, T, m->total_chunks, m->chunk_tokens, c.max_blocks_per_seq, c.n_pool_blocks, c.n_heads,
+                                                         c.n_kv_heads, D, s), "paged_attention_decode");
+      m->launches += 2;
+      LG_TRY(few_act(m->attn.p, H, L.wo, m->x.p, T, H, LG_EPI_RESID_F32, &m->launches, s), "output projection of few rows");
+      LG_TRY(few_norm(m->x, L.norm2, c.rms_eps, L.wgu, nullptr, m->act.p, T, I, LG_EPI_SWIGLU, &m->launches, s), "norm and gate/up of few rows");
+      LG_TRY(few_act(m->act.p, I, L.wdown, m->x.p, T, H, LG_EPI_RESID_F32, &m->launches, s), "down projection of few rows");
+      continue;
+    }
     LG_TRY(logismos_launch_rms_norm_f32(m->x.p, L.norm1.p, m->h.p, T, H, c.rms_eps, 0, s), "rms_norm");
     if (uint32_t rc = qlinear(m, m->h.p, L.wqkv, L.bqkv.p, m->qkv.p, T, H, QKV, LG_EPI_BF16, s)) return rc;
     LG_TRY(logismos_launch_rope_halves_bf16(m->qkv.p, m->cos.p, m->sin.p, m->pos.p, T, c.n_heads + c.n_kv_heads, D, QKV,
@@ -221,7 +235,7 @@ uint32_t lg_decoder_create(int32_t device, const lg_decoder_config_t* cfg, const
   size_t wmax = QKV * H;
   if (2 * I * H > wmax) wmax = 2 * I * H;
   // every sequence of a step may be a decode sequence of up to max_blocks_per_seq blocks
-  m->max_chunks = S * ((MB * kBlock + kChunkTokens - 1) / kChunkTokens);
+  m->max_chunks = std::max(kMinDecodeChunks, S * ((MB * kBlock + kChunkTokens - 1) / kChunkTokens));
   const size_t acc_n = QKV > 2 * I ? QKV : 2 * I;
   ok = ok && m->x.alloc(T * H * 4) && m->h.alloc(T * H * 2) && m->qkv.alloc(T * QKV * 2) && m->attn.alloc(T * H * 2) &&
        m->qdec.alloc(S * H * 2) && m->gu.alloc(16) && m->act.alloc(T * I * 2) && m->wscratch.alloc(wmax * 2) &&
@@ -294,7 +308,7 @@ uint32_t lg_decoder_step(void* model, const uint32_t* host_ids, const int32_t* c
   const int n_dec = B.n_dec;
   const bool has_prefix = B.has_prefix;
   const size_t total = (size_t)B.T;
-  m->chunk_tokens = n_dec > 0 ? logismos_pick_decode_chunk(B.ctx, n_dec, m->cfg.n_kv_heads, m->head_dim) : kChunkTokens;
+  m->chunk_tokens = n_dec > 0 ? step_decode_chunk(B.ctx, n_dec, m->cfg.n_kv_heads, m->head_dim, m->max_chunks) : kChunkTokens;
   const int total_chunks = n_dec > 0 ? logismos_build_decode_chunks(B.ctx, n_dec, m->chunk_tokens, B.chunks) : 0;
   if (total_chunks < 0 || (size_t)total_chunks > m->max_chunks) { set_error("lg_decoder_step: decode chunk count exceeds the scratch"); return LG_EMB_COMPUTE; }
   m->T = B.T; m->n_dec = n_dec; m->n_pre = B.n_pre; m->n_seqs = n_seqs; m->max_pre_len = B.max_pre_len; m->total_chunks = total_chunks;

@@ -118,8 +118,33 @@ uint32_t run_device(Hybrid* m, cudaStream_t s) {
   }
   LG_TRY(logismos_launch_embed_lookup_bf16(m->tok_embed.p, m->ids.p, m->x.p, T, H, c.vocab, s), "embed_lookup");
   m->launches += 1;
+  const bool few = m->n_pre == 0 && lg::int4_rows_fit(T, std::max({H, I, QW, GW})) && !m->allreduce && !m->reduce_add;
   for (int l = 0; l < c.n_layers; ++l) {
     HLayer& L = m->layers[l];
+    if (few) {
+      if (L.full) {  // columns: q | k | v | gate
+        const lg::DecodeHeads heads{D, c.n_heads, c.n_kv_heads, c.max_pos, (const float*)m->cos.p, (const float*)m->sin.p, (const int*)m->pos.p, (const int64_t*)m->slots.p,
+                                    (int64_t)c.n_pool_blocks * kBlock, (__nv_bfloat16*)m->qdec.p, (__nv_bfloat16*)L.kpool.p, (__nv_bfloat16*)L.vpool.p,
+                                    (__nv_bfloat16*)m->proj.p + QW + 2 * KW, AN, (int*)st};
+        LG_TRY(few_heads(m->x, L.norm1, c.rms_eps, L.w_in, nullptr, heads, T, &m->launches, s), "norm, projections, rope and cache store of few rows");
+        LG_TRY(logismos_launch_paged_attention_decode_bf16(m->qdec.p, L.kpool.p, L.vpool.p, nullptr, nullptr, m->dec_tables.p, m->dec_ctx.p, m->dec_chunks.p, m->mix.p,
+                                                           m->dec_scratch.p, st, T, m->total_chunks, m->chunk_tokens, c.max_blocks_per_seq, c.n_pool_blocks, c.n_heads,
+                                                           c.n_kv_heads, D, s), "paged_attention_decode");
+        LG_TRY(logismos_launch_gated_mul_bf16(m->mix.p, QW, (uint16_t*)m->proj.p + QW + 2 * KW, AN, T, QW, 0, s), "attention gate");
+        m->launches += 3;
+        LG_TRY(few_act(m->mix.p, QW, L.w_out, m->x.p, T, H, LG_EPI_RESID_F32, &m->launches, s), "output projection of few rows");
+      } else {  // columns: q | k | v | z | a | b, whose fp32 sums the recurrence takes (and leaves zero)
+        const int ld = GN + 2 * GH;
+        LG_TRY(few_norm(m->x, L.norm1, c.rms_eps, L.w_in, nullptr, m->accws.p, T, ld, LG_EPI_F32, &m->launches, s), "norm and projections of few rows");
+        LG_TRY(logismos_launch_gdn_decode_from_acc(L.state.p, m->accws.p, ld, L.A_log.p, L.dt_bias.p, m->mix.p, m->state_slots.p, m->fresh.p, m->gdn_pairs.p, m->n_dec, GH,
+                                                   1.0f / std::sqrt((float)kGdnDim), s), "gdn decode from the projections' sums");
+        m->launches += 1;
+        LG_TRY(few_act(m->mix.p, GW, L.w_out, m->x.p, T, H, LG_EPI_RESID_F32, &m->launches, s), "output projection of few rows");
+      }
+      LG_TRY(few_norm(m->x, L.norm2, c.rms_eps, L.wgu, nullptr, m->act.p, T, I, LG_EPI_SWIGLU, &m->launches, s), "norm and gate/up of few rows");
+      LG_TRY(few_act(m->act.p, I, L.wdown, m->x.p, T, H, LG_EPI_RESID_F32, &m->launches, s), "down projection of few rows");
+      continue;
+    }
     LG_TRY(logismos_launch_rms_norm_f32(m->x.p, L.norm1.p, m->h.p, T, H, c.rms_eps, 0, s), "rms_norm");
     m->launches += 1;
     uint16_t* p16 = (uint16_t*)m->proj.p;
@@ -330,7 +355,7 @@ uint32_t lg_hybrid_create(int32_t device, const lg_hybrid_config_t* cfg, const l
   size_t wmax = pn * H;
   if ((size_t)2 * I * H > wmax) wmax = (size_t)2 * I * H;
   if ((size_t)m->mix_w * H > wmax) wmax = (size_t)m->mix_w * H;
-  m->max_chunks = S * ((MB * kBlock + kChunkTokens - 1) / kChunkTokens);
+  m->max_chunks = std::max(kMinDecodeChunks, S * ((MB * kBlock + kChunkTokens - 1) / kChunkTokens));
   const size_t acc_n = pn + 2 * GH > (size_t)2 * I ? pn + 2 * GH : (size_t)2 * I;
   ok = ok && m->x.alloc(T * H * 4) && m->delta.alloc(T * H * 4) && m->h.alloc(T * H * 2) && m->proj.alloc(T * pn * 2) && m->mix.alloc(T * m->mix_w * 2) &&
        m->qdec.alloc(S * QW * 2) && m->ab.alloc(T * 2 * GH * 4) && m->g.alloc(T * GH * 4) && m->beta.alloc(T * GH * 4) &&
@@ -405,7 +430,7 @@ uint32_t lg_hybrid_step(void* model, const uint32_t* host_ids, const int32_t* ca
   const int n_dec = B.n_dec, n_pre = B.n_pre;
   const bool has_prefix = B.has_prefix;
   const size_t total = (size_t)B.T;
-  m->chunk_tokens = n_dec > 0 ? logismos_pick_decode_chunk(B.ctx, n_dec, m->cfg.n_kv_heads, m->cfg.attn_head_dim) : kChunkTokens;
+  m->chunk_tokens = n_dec > 0 ? step_decode_chunk(B.ctx, n_dec, m->cfg.n_kv_heads, m->cfg.attn_head_dim, m->max_chunks) : kChunkTokens;
   const int total_chunks = n_dec > 0 ? logismos_build_decode_chunks(B.ctx, n_dec, m->chunk_tokens, B.chunks) : 0;
   if (total_chunks < 0 || (size_t)total_chunks > m->max_chunks) { set_error("lg_hybrid_step: decode chunk count exceeds the scratch"); return LG_EMB_COMPUTE; }
   m->T = B.T; m->n_dec = n_dec; m->n_pre = n_pre; m->n_seqs = n_seqs; m->max_pre_len = B.max_pre_len; m->total_chunks = total_chunks;

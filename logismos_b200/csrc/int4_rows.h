@@ -1,0 +1,44 @@
+// The decode steps of one to four rows: int4 projections with the norm in front and what follows behind them in one launch, down
+// to the rotation and the cache store of their heads (int4_rows.cu).
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace lg {
+
+constexpr int kFewRows = 4;  // the most rows of a launch: see int4_rows.cu
+
+// Columns that are heads: q heads rotated to q_out [rows][n_heads * dim], k heads rotated and v heads to their cache slots, further
+// heads to rest [rows][ld_rest].
+struct DecodeHeads {
+  int dim, n_heads, n_kv, max_pos;  // dim 0: none
+  const float *cos, *sin;           // [max_pos][dim / 2]
+  const int* positions;
+  const int64_t* slots;
+  int64_t n_slots;
+  __nv_bfloat16 *q_out, *k_pool, *v_pool, *rest;
+  int ld_rest;
+  int* status;
+};
+
+struct Int4Rows {
+  // activations: the fp32 residual stream [rows][k] with the gain of its RMS norm, or bf16 [rows][lda]
+  const void* x;
+  const void* gain;
+  float eps;
+  const void* a;
+  int lda;
+  const void *codes, *scales, *bias;
+  void* out;
+  int rows, n, k, ldc;
+  int epi;  // LG_EPI_BF16, LG_EPI_RESID_F32 (in place), LG_EPI_SWIGLU or LG_EPI_F32 (stored)
+  DecodeHeads heads;  // dim > 0: in place of out and epi
+};
+
+// what the activations of a launch take of shared memory
+inline bool int4_rows_fit(int rows, int k) { return rows >= 1 && rows <= kFewRows && k > 0 && k % 128 == 0 && (size_t)rows * (k + 32) * 2 + (size_t)k <= 200 * 1024; }
+bool int4_rows_takes(const Int4Rows& p);
+uint32_t launch_int4_rows(const Int4Rows& p, cudaStream_t stream);
+
+}  // namespace lg

@@ -10,6 +10,7 @@
 #include <thread>
 #include <vector>
 
+#include "int4_rows.h"
 #include "logismos_kernels.h"
 #include "logismos_model.h"
 
@@ -194,6 +195,49 @@ inline uint32_t qlinear_any(const void* a, const QMat& w, const void* bias, void
   *launches += 2;
   return logismos_launch_linear_t_bf16(a, wscratch, bias, out, T, w.n, w.k, lda, ldc, epi, status, s);
 }
+
+// The projections of a pure decode step of one to four rows (int4_rows.cu). norm: x is the fp32 residual stream and goes
+// through its RMS norm on the way; otherwise a is bf16 activations with row stride lda.
+inline lg::Int4Rows few_rows(const QMat& w, const void* bias, void* out, int rows, int ldc, int epi) {
+  lg::Int4Rows p{};
+  p.codes = w.codes.p; p.scales = w.scales.p; p.bias = bias; p.out = out;
+  p.rows = rows; p.n = w.n; p.k = w.k; p.ldc = ldc; p.epi = epi;
+  return p;
+}
+inline uint32_t few_norm(const Buf& x, const Buf& gain, float eps, const QMat& w, const void* bias, void* out, int rows, int ldc, int epi, int* launches, cudaStream_t s) {
+  lg::Int4Rows p = few_rows(w, bias, out, rows, ldc, epi);
+  p.x = x.p; p.gain = gain.p; p.eps = eps;
+  *launches += 1;
+  return lg::launch_int4_rows(p, s);
+}
+inline uint32_t few_heads(const Buf& x, const Buf& gain, float eps, const QMat& w, const void* bias, const lg::DecodeHeads& heads, int rows, int* launches, cudaStream_t s) {
+  lg::Int4Rows p = few_rows(w, bias, nullptr, rows, 0, LG_EPI_BF16);
+  p.x = x.p; p.gain = gain.p; p.eps = eps; p.heads = heads;
+  *launches += 1;
+  return lg::launch_int4_rows(p, s);
+}
+inline uint32_t few_act(const void* a, int lda, const QMat& w, void* out, int rows, int ldc, int epi, int* launches, cudaStream_t s) {
+  lg::Int4Rows p = few_rows(w, nullptr, out, rows, ldc, epi);
+  p.a = a; p.lda = lda;
+  *launches += 1;
+  return lg::launch_int4_rows(p, s);
+}
+
+// Tokens per decode chunk of a step: logismos_pick_decode_chunk's, and shorter where that leaves most SMs without a CTA
+// (one sequence of 1200 tokens, two key heads of 128: 6 CTAs of 512 tokens 14.5 us, 20 of 128 8.8 us), as far as the
+// scratch holds the partial results.
+inline int step_decode_chunk(const int32_t* ctx, int n_dec, int n_kv_heads, int head_dim, size_t max_chunks) {
+  int chunk = logismos_pick_decode_chunk(ctx, n_dec, n_kv_heads, head_dim);
+  if (chunk > 512) return chunk;
+  auto count = [&](int c) {
+    int64_t n = 0;
+    for (int i = 0; i < n_dec; ++i) n += (std::max(ctx[i], 1) + c - 1) / c;
+    return n;
+  };
+  while (chunk > 128 && count(chunk) * n_kv_heads < 148 && count(chunk / 2) <= (int64_t)max_chunks) chunk /= 2;
+  return chunk;
+}
+constexpr size_t kMinDecodeChunks = 1024;  // partial results that a model's scratch holds at least
 
 // logits = hidden W^T over the vocabulary and decode::greedy (crates/decode/src/lib.rs:73-83) on
 // them. The logits stay fp32 up to the argmax on every route, as in the reference (greedy takes the

@@ -124,3 +124,31 @@ def test_turbo3_cache_mode_runs_the_same_steps_at_the_codec_accuracy(setup):
             assert np.isfinite(hs[row]).all() and cosine(hs[row], h_ref) >= 0.9, (sid, cosine(hs[row], h_ref))
         hist[0].append(int(toks[0])); hist[1].append(int(toks[1]))
     model.close()
+
+
+@pytest.mark.parametrize("n_seqs", [1, 2, 3, 4, 5])
+def test_decode_steps_of_few_sequences(n_seqs):
+    """Up to four rows the projections run as one launch each with the norm in front and rotation, cache store or SwiGLU behind;
+    five rows take the general route. Widths that leave uneven slices of k (20 and 44 groups of 32), contexts on both sides
+    of a decode chunk."""
+    cfg = dict(TINY, hidden=640, n_heads=5, n_kv_heads=1, intermediate=1408, vocab=700)
+    w = make_weights(cfg, 31)
+    qw, deq = quantize_weights(cfg, w)
+    oracle = O.OracleStella(cfg, deq)
+    rng = np.random.default_rng(n_seqs)
+    alloc = BlockAllocator(128, 32, seed=3)
+    model = DecoderModel(cfg, qw, n_pool_blocks=128, max_blocks_per_seq=32, max_step_tokens=512, max_step_seqs=9)
+    lens = [127, 40, 16, 1, 130, 3, 20, 8, 5][:n_seqs]
+    hist = [rng.integers(0, cfg["vocab"], n).tolist() for n in lens]
+    toks = model.step(sum(hist, []), [0] * n_seqs, lens, np.stack([alloc.ensure(i, n) for i, n in enumerate(lens)]))
+    for _ in range(3):
+        for i in range(n_seqs):
+            hist[i].append(int(toks[i]))
+        toks = model.step([h[-1] for h in hist], [len(h) - 1 for h in hist], [1] * n_seqs, np.stack([alloc.ensure(i, len(h)) for i, h in enumerate(hist)]))
+        assert model.device_status() == 0
+        hs, lg = model.last_hidden(), model.last_logits()
+        for i, ids in enumerate(hist):
+            h_ref = oracle.forward(np.asarray(ids, np.uint32), causal=True)[-1]
+            assert max_rel(hs[i], h_ref) <= TOL and max_rel(lg[i], O.linear_t(h_ref, deq["lm_head"], None, 1, cfg["vocab"], cfg["hidden"])) <= TOL, i
+            assert toks[i] == O.greedy(lg[i])
+    model.close()
