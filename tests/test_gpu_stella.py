@@ -144,3 +144,21 @@ def test_full_size_stella_1_5b_parity_on_short_sequences():
     emb_p = m.encode_ids_batch(ids_p, cu_p)
     assert np.abs(emb_p - emb[order]).max() < 1e-4
     m.close()
+
+
+@pytest.mark.parametrize("lens", [[17], [1], [64, 1, 33], [32, 32, 32, 32], [5] * 20, [63, 2, 62], [65], [64, 64, 1]])
+def test_short_texts(lens):
+    """Batches of up to 128 tokens with texts of up to 64 take fp32 sums of the q, k, v projection straight into their attention: both
+    lane widths (32 and 64 keys), single tokens, a full batch; 65 tokens in a text or 129 in the batch take the general route."""
+    cfg = dict(TINY, n_layers=3)
+    w = make_weights(cfg, 5)
+    model = StellaModel(cfg, w, max_batch_tokens=256, max_batch_seqs=32)
+    oracle = O.OracleStella(cfg, w)
+    cu = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ids = np.random.default_rng(sum(lens)).integers(0, cfg["vocab"], int(cu[-1]), dtype=np.uint32)
+    for _ in range(2):   # the second time over buffers that the first left
+        got = model.encode_ids_batch(ids, cu)
+        ref = oracle.encode_batch(ids, cu, 4)
+        assert model.device_status() == 0
+        assert min(float((a * b).sum()) for a, b in zip(got, ref)) >= 0.9999 and np.abs(got - ref).max() <= 2e-2 * np.abs(ref).max()
+    model.close()
