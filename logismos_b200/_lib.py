@@ -106,6 +106,7 @@ def _declare(l, partial=False):
         "logismos_launch_min_p_f32": [vp, i32, i32, f32, vp],
         "logismos_launch_repetition_penalty_f32": [vp, i32, i32, vp, vp, i32, f32, vp],
         "logismos_launch_multinomial_f32": [vp, i32, i32, vp, vp, vp],
+        "logismos_launch_sample_chain_f32": [vp, i32, i32, f32, i32, f32, f32, vp, vp, vp],
         # model
         "logismos_launch_quantize_int4_g32": [vp, vp, vp, i32, i32, vp],
         "lg_safetensors_open": [C.c_char_p, C.POINTER(vp)],

@@ -1,7 +1,7 @@
 // The sampling chain on the device: the logit processors and the multinomial sampler of the
 // reference's decode crate over fp32 logits [rows, n] (n = 151936 for the decoder configurations),
 // in place, one launch per processor so that a chain keeps the reference's free ordering
-// (crates/decode/src/chain.rs:33-76):
+// (crates/decode/src/chain.rs:33-76), or one launch for the usual order with a small k (few_survivors_kernel):
 //   TemperatureScale    crates/decode/src/processors.rs:18-28
 //   TopK                :50-82     (k-th largest by radix select on the float bits: exact)
 //   TopP                :89-122    (smallest prefix by descending probability whose mass reaches p)
@@ -12,7 +12,7 @@
 // order-preserving integer key of the logit, 11 bits per pass (three passes of 2048 bins). One CTA per row left most of the
 // chip idle; a row is a cluster of eight CTAs that meet through each other's shared memory (rows below kClusterFrom
 // values: one CTA). What bounds them is the work that does not shrink with the slice, barriers and the reduction of the
-// bins, so a CTA has 256 threads (64 x 151936, TopK: 49 us; 512 threads 57, 1024 threads with the slice held in
+// bins, so a CTA has 256 threads (64 x 151936, TopK by radix select: 49 us; 512 threads 57, 1024 threads with the slice held in
 // shared memory 75) and goes over its slice as rarely as it can: values that can still hold the cut, or all that TopK has left,
 // are listed in shared memory, and later passes go over the list. Bins hold integers, counts and probabilities in units of
 // 2^-40 (2^-56 in rows above 262 thousand values: one below half a unit has no mass), so shared-memory atomics give the same sums in any order and results do not change between runs. Ties
@@ -37,6 +37,14 @@ static_assert(kSegment == kThreads, "a thread per bin of a segment");
 // rows: 2500 values 24 us either way, 4001 28 as one CTA and 27 as a cluster, 8000 42 and 31).
 constexpr int kClusterFrom = 2048;
 constexpr int kListed = 1024;     // values that a CTA can list
+// few_survivors_kernel: the largest k, and the most values that it may find above its bound. Of 2048 shares, k = 256 of them hold the
+// 273 largest values on average, so twice k leaves room for values that lie together.
+constexpr int kFewK = 256, kFound = 512;
+static_assert(2 * kFound <= kListed && kMaxCluster * kThreads <= 2 * kBins, "found values twice in the list, a key per thread in the bins");
+
+// Masses are counted in units of 2^-(24 + bits): 2^-40 as long as the sums of a slice's low words fit 32 bits (262 thousand values); longer rows, whose
+// probabilities are smaller, in units of 2^-56 with carries.
+LG_DEVINL int mass_bits(int n, int size) { return (n + size - 1) / size + 4 < 32768 ? 16 : 32; }
 
 // larger float <-> larger key; NaN is ordered like -inf (TopK folds NaN to -inf before its sort)
 LG_DEVINL uint32_t order_key(float v) {
@@ -396,14 +404,7 @@ LG_DEVINL void mask_below_cut(const cg::cluster_group& c, const Row& row, uint32
 
 // A CTA may not leave while another still reads its shared memory: every kernel ends with a barrier of the cluster.
 
-// 170 -> 49 us on 64 x 151936, k = 50
-__global__ void __launch_bounds__(kThreads, 4)
-top_k_kernel(float* __restrict__ logits, int n, int k) {
-  __shared__ uint32_t bins[kBins];
-  __shared__ int2 room[kListed];
-  __shared__ Shared sh;
-  const cg::cluster_group c = cg::this_cluster();
-  Row row(logits, n, c);
+__device__ __noinline__ void top_k_row(const cg::cluster_group& c, Row row, int k, uint32_t* bins, int2* room, Shared& sh) {
   row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
   const uint32_t cut = radix_select<false>(c, row, 0.0f, 0.0f, 0ull, (uint32_t)k, 0, bins, room, sh);
   row.list = nullptr;
@@ -412,22 +413,13 @@ top_k_kernel(float* __restrict__ logits, int n, int k) {
   row_sync(c, row);
 }
 
-// 186 -> 36 us on 64 x 151936 after top-k 50, 215 -> 100 us on whole rows
-__global__ void __launch_bounds__(kThreads, 4)
-top_p_kernel(float* __restrict__ logits, int n, float p) {
-  __shared__ uint32_t bins[2 * kBins];
-  __shared__ int2 room[kListed];
-  __shared__ Shared sh;
-  const cg::cluster_group c = cg::this_cluster();
-  Row row(logits, n, c);
+__device__ __noinline__ void top_p_row(const cg::cluster_group& c, Row row, float p, uint32_t* bins, int2* room, Shared& sh) {
   row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
   float mx, sum;
   row_max_sum(c, row, false, room, sh, mx, sum);
   const bool whole = row.list != nullptr;  // the list has all that is above -inf: nothing else is to be masked
   const float inv = sum > 0.0f ? 1.0f / sum : 1.0f;
-  // units of 2^-40 as long as the sums of a slice's low words fit 32 bits (262 thousand values); longer rows, whose probabilities are
-  // smaller, in units of 2^-56 with carries
-  const int slice = (n + row.size - 1) / row.size + 4, lo_bits = slice < 32768 ? 16 : 32;
+  const int lo_bits = mass_bits(row.n, row.size);
   const float unit = ldexpf(1.0f, 24 + lo_bits);
   const unsigned long long target = (unsigned long long)ceil((double)p * (double)unit);
   const bool finite = fabsf(mx) <= 3.402823466e38f;
@@ -449,13 +441,7 @@ top_p_kernel(float* __restrict__ logits, int n, float p) {
   row_sync(c, row);
 }
 
-// 53 -> 39 us on 64 x 151936
-__global__ void __launch_bounds__(kThreads, 4)
-min_p_kernel(float* __restrict__ logits, int n, float p) {
-  __shared__ int2 room[kListed];
-  __shared__ Shared sh;
-  const cg::cluster_group c = cg::this_cluster();
-  Row row(logits, n, c);
+__device__ __noinline__ void min_p_row(const cg::cluster_group& c, Row row, float p, int2* room, Shared& sh) {
   row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
   float mx, sum;
   row_max_sum(c, row, false, room, sh, mx, sum);
@@ -473,16 +459,11 @@ min_p_kernel(float* __restrict__ logits, int n, float p) {
 // MultinomialSampler::sample for a given uniform draw. The reference walks the row (u < p_i returns i, else u -= p_i);
 // here a CTA owns a contiguous slice, each warp a part of it and each chunk of at least 128 values a part of that. Masses are
 // summed per chunk; the warp whose part holds the draw finds its chunk and walks on from there 32 values at a time
-// (whole parts walked: one load's latency per 32 values). A value without mass is never drawn. 88 -> 35 us on 64 x 151936 after top-k 50
-__global__ void __launch_bounds__(kThreads, 4)
-multinomial_kernel(const float* __restrict__ logits, int n, const float* __restrict__ uniforms, uint32_t* __restrict__ out) {
+// (whole parts walked: one load's latency per 32 values). A value without mass is never drawn.
+__device__ __noinline__ void multinomial_row(const cg::cluster_group& c, Row row, const float* uniforms, uint32_t* out, int2* room, Shared& sh) {
   constexpr int kWarps = kThreads / 32;
-  __shared__ int2 room[kListed];
-  __shared__ Shared sh;
   __shared__ float s_chunk[kWarps][32], s_mass[kWarps];
-  const cg::cluster_group c = cg::this_cluster();
-  Row row(const_cast<float*>(logits), n, c);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, out_row = blockIdx.x / row.size;
+  const int n = row.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, out_row = blockIdx.x / row.size;
   if (threadIdx.x == 0) sh.best = 0xffffffffu;
   row_sync(c, row);  // every CTA of the row runs, so its shared memory may be written
   float mx, sum;
@@ -573,6 +554,272 @@ multinomial_kernel(const float* __restrict__ logits, int n, const float* __restr
   if (row.rank == 0 && threadIdx.x == 0) out[out_row] = sh.best == 0xffffffffu ? (uint32_t)(n - 1) : u < total ? sh.best : (uint32_t)(n - 1) - sh.best;
 }
 
+
+// 215 -> 100 us on 64 x 151936, 36 after a top-k of 50
+__global__ void __launch_bounds__(kThreads, 4)
+top_p_kernel(float* __restrict__ logits, int n, float p) {
+  __shared__ uint32_t bins[2 * kBins];
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  const cg::cluster_group c = cg::this_cluster();
+  top_p_row(c, Row(logits, n, c), p, bins, room, sh);
+}
+
+// 53 -> 39 us on 64 x 151936
+__global__ void __launch_bounds__(kThreads, 4)
+min_p_kernel(float* __restrict__ logits, int n, float p) {
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  const cg::cluster_group c = cg::this_cluster();
+  min_p_row(c, Row(logits, n, c), p, room, sh);
+}
+
+// 88 -> 35 us on 64 x 151936 after top-k 50
+__global__ void __launch_bounds__(kThreads, 4)
+multinomial_kernel(const float* __restrict__ logits, int n, const float* __restrict__ uniforms, uint32_t* __restrict__ out) {
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  const cg::cluster_group c = cg::this_cluster();
+  multinomial_row(c, Row(const_cast<float*>(logits), n, c), uniforms, out, room, sh);
+}
+
+// for k above kFewK
+__global__ void __launch_bounds__(kThreads, 4)
+top_k_kernel(float* __restrict__ logits, int n, int k) {
+  __shared__ uint32_t bins[kBins];
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  const cg::cluster_group c = cg::this_cluster();
+  top_k_row(c, Row(logits, n, c), k, bins, room, sh);
+}
+
+// Temperature, top-k with few survivors and what a chain does with these.
+struct Chain {
+  float temperature;      // 1: none
+  int k;                  // 1 .. kFewK, below n
+  float p, min_p;         // p >= 1, min_p <= 0: none
+  const float* uniforms;  // null: no draw
+  uint32_t* out;
+};
+
+// Sums of the masses of list[0 .. m) as row_max_sum leaves them: integers per slice, fp32 over the slices. Every thread gets the sum.
+LG_DEVINL float survivor_sum(const int2* list, int m, int n, int size, float mx, bool finite_only, unsigned long long* seg, uint32_t* nan) {
+  const int per = ((n + size - 1) / size + 3) & ~3;
+  __syncthreads();
+  if (threadIdx.x < kMaxCluster) { seg[threadIdx.x] = 0; nan[threadIdx.x] = 0; }
+  __syncthreads();
+  for (int j = threadIdx.x; j < m; j += kThreads) {
+    const float v = __int_as_float(list[j].y), e = finite_only && !(fabsf(v) <= 3.402823466e38f) ? 0.0f : expf(v - mx);
+    if (e != e) nan[list[j].x / per] = 1;
+    else atomicAdd(seg + list[j].x / per, __float2ull_rn(e * 1125899906842624.0f));
+  }
+  __syncthreads();
+  float sum = 0.0f;
+  for (int r = 0; r < size; ++r) sum += nan[r] ? NAN : (float)seg[r] * (1.0f / 1125899906842624.0f);
+  return sum;
+}
+
+// One launch for temperature, top-k, top-p, min-p and the draw, where k is small: after top-k the rest of the chain has k values to look at
+// and no row. What bounds it is one read and one write of the rows. The read leaves each thread the maximum of its
+// share; the k-th largest of the row's 2048 maxima is a lower bound of its k-th largest value (k shares hold a value that
+// large), few values lie above it, and only the threads whose maximum does go over their share again. The values found
+// go to the first CTA of the row, which orders them by value (ties by index) and finishes the chain while all CTAs set the row to -inf; then it
+// puts the survivors back. Division by the temperature keeps the order, so only maxima, bounds and the values found are divided.
+// A row with more values above the bound than kFound (many ties) goes through the general functions. Masses and sums are
+// formed as these form them, so the survivors are the same. 64 x 151936, temperature, k = 50, p = 0.95 and the draw: 25 us (39 MB read and written, 12 us at
+// the copy rate) against 136 in four launches; top-k alone 53 before.
+__global__ void __launch_bounds__(kThreads, 4)
+few_survivors_kernel(float* __restrict__ logits, int n, const Chain ch) {
+  __shared__ __align__(16) uint32_t bins[2 * kBins];
+  __shared__ int2 room[kListed];
+  __shared__ Shared sh;
+  __shared__ uint32_t s_count[32], s_found, s_nan[kMaxCluster];
+  const cg::cluster_group c = cg::this_cluster();
+  const Row row(logits, n, c);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool divide = ch.temperature != 1.0f;
+  auto scaled = [&](float v) { return divide ? v / ch.temperature : v; };
+  // 16-byte pieces of the row, the first and the last one perhaps in part; piece q holds values 4 q - lead ..
+  const int lead = (int)((reinterpret_cast<uintptr_t>(row.l) >> 2) & 3), pieces = (lead + n + 3) >> 2, per = (pieces + row.size - 1) / row.size;
+  const int q0 = min(row.rank * per, pieces), q1 = min(q0 + per, pieces);
+  float* const first = row.l - lead;
+  auto whole = [&](int q) { return 4 * q >= lead && 4 * q + 4 <= lead + n; };
+  auto load = [&](int q) {  // a partial one
+    const int i = 4 * q - lead;
+    auto at = [&](int j) { return j >= 0 && j < n ? row.l[j] : -INFINITY; };
+    return make_float4(at(i), at(i + 1), at(i + 2), at(i + 3));
+  };
+  // the pieces of this slice that are whole; what is left of it is the row's first or last piece
+  const int w0 = q0 == 0 && lead && q1 > q0 ? 1 : q0, w1 = q1 == pieces && q1 > q0 && !whole(pieces - 1) ? max(q1 - 1, w0) : q1;
+  if (tid < 32) s_count[tid] = 0;
+  if (tid == 0) s_found = 0;
+  c.barrier_arrive();  // every CTA of the row runs once this is passed, so its shared memory may be written
+  float m = -INFINITY;
+  auto larger = [&](float4 v) { m = fmaxf(m, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w))); };  // fmaxf drops NaN, which top-k takes for -inf
+#pragma unroll 8
+  for (int q = w0 + tid; q < w1; q += kThreads) larger(*reinterpret_cast<const float4*>(first + 4 * (size_t)q));
+  // the partial pieces belong to the last two threads
+  const int part = tid == kThreads - 1 && w0 > q0 ? q0 : tid == kThreads - 2 && w1 < q1 ? q1 - 1 : -1;
+  if (part >= 0) larger(load(part));
+  c.barrier_wait();
+  uint32_t* const keys = bins;  // [size][kThreads]
+  const uint32_t own_key = order_key(m);
+  for (int r = 0; r < row.size; ++r) c.map_shared_rank(keys, r)[row.rank * kThreads + tid] = own_key;
+  row_sync(c, row);
+  uint32_t held[kMaxCluster];
+  for (int r = 0; r < kMaxCluster; ++r) held[r] = r < row.size ? keys[r * kThreads + tid] : 0u;
+  uint32_t bound = 0;  // the leading 16 bits of the k-th largest maximum, two at a time
+#pragma unroll 1
+  for (int bit = 30; bit >= 16; bit -= 2) {
+    const uint32_t step = 1u << bit;
+    uint32_t c12 = 0, c3 = 0;
+#pragma unroll
+    for (int r = 0; r < kMaxCluster; ++r) {
+      c12 += (held[r] >= bound + step ? 1u : 0u) + (held[r] >= bound + 2 * step ? 0x10000u : 0u);
+      c3 += held[r] >= bound + 3 * step ? 1u : 0u;
+    }
+    c12 = __reduce_add_sync(0xffffffffu, c12);
+    c3 = __reduce_add_sync(0xffffffffu, c3);
+    if (lane == 0) {
+      if (c12) atomicAdd(s_count + bit, c12);
+      if (c3) atomicAdd(s_count + bit + 1, c3);
+    }
+    __syncthreads();
+    const uint32_t n12 = s_count[bit], n3 = s_count[bit + 1], k = (uint32_t)ch.k;
+    bound += n3 >= k ? 3 * step : (n12 >> 16) >= k ? 2 * step : (n12 & 0xffffu) >= k ? step : 0u;
+  }
+  // at and below -inf (whose truncated key would be a NaN) every number counts
+  const float low = bound <= 0x007fffffu ? -INFINITY : scaled(__uint_as_float(bound & 0x80000000u ? bound & 0x7fffffffu : ~bound));
+  uint32_t* const found = c.map_shared_rank(&s_found, 0);
+  int2* const list = c.map_shared_rank(room, 0);
+  auto above = [&](float v) { return v >= low && v > -INFINITY; };
+  auto look = [&](int q, float4 v) {
+    const float w[4] = {scaled(v.x), scaled(v.y), scaled(v.z), scaled(v.w)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (!above(w[j])) continue;
+      const uint32_t at = atomicAdd(found, 1u);
+      if (at < (uint32_t)kFound) list[at] = make_int2(4 * q + j - lead, __float_as_int(w[j]));
+    }
+  };
+  const bool has = above(scaled(m));
+  if (has && part >= 0) look(part, load(part));
+  // the lanes of a warp go over the share of each of them that has something, one round of loads for 32 pieces
+  for (uint32_t lanes = __ballot_sync(0xffffffffu, has); lanes; lanes &= lanes - 1) {
+    const int whose = w0 + (tid & ~31) + __ffs(lanes) - 1;
+    for (int q = whose + lane * kThreads; q < w1; q += 32 * kThreads) look(q, *reinterpret_cast<const float4*>(first + 4 * (size_t)q));
+  }
+  row_sync(c, row);
+  const uint32_t total = *found;
+  if (total > (uint32_t)kFound) {
+    if (divide) {
+      for (int i = row.begin + tid; i < row.end; i += kThreads) row.l[i] = row.l[i] / ch.temperature;
+    }
+    top_k_row(c, row, ch.k, bins, room, sh);
+    if (ch.p < 1.0f) top_p_row(c, row, ch.p, bins, room, sh);
+    if (ch.min_p > 0.0f) min_p_row(c, row, ch.min_p, room, sh);
+    if (ch.uniforms) multinomial_row(c, row, ch.uniforms, ch.out, room, sh);
+    return;
+  }
+  const float4 none = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+#pragma unroll 4
+  for (int q = w0 + tid; q < w1; q += kThreads) *reinterpret_cast<float4*>(first + 4 * (size_t)q) = none;
+  if (part >= 0)
+    for (int i = max(4 * part - lead, 0); i < min(4 * part + 4 - lead, n); ++i) row.l[i] = -INFINITY;
+  int kept = 0;
+  int2* const sorted = room + kFound;  // by value, ties by index
+  if (row.rank == 0) {
+    const int count = (int)total;
+    for (int j = tid; j < count; j += kThreads) {
+      const int2 e = room[j];
+      const uint32_t key = order_key(__int_as_float(e.y));
+      int rank = 0;
+      for (int i = 0; i < count; ++i) {
+        const int2 o = room[i];
+        const uint32_t other = order_key(__int_as_float(o.y));
+        rank += other > key || (other == key && o.x < e.x) ? 1 : 0;
+      }
+      sorted[rank] = e;
+    }
+    __syncthreads();
+    auto value = [&](int j) { return __int_as_float(sorted[j].y); };
+    auto leading = [&](auto&& keep) {  // how many of the kFound first hold
+      int k = 0;
+#pragma unroll
+      for (int j0 = 0; j0 < kFound; j0 += kThreads) k += __syncthreads_count(j0 + tid < kept && keep(j0 + tid));
+      return k;
+    };
+    unsigned long long* const seg = sh.seg;
+    kept = count;
+    if (count > ch.k) {
+      const uint32_t cut = order_key(value(ch.k - 1));  // what ties with the k-th largest survives
+      kept = leading([&](int j) { return order_key(value(j)) >= cut; });
+    }
+    const float mx = kept ? value(0) : -INFINITY;
+    if (ch.p < 1.0f && fabsf(mx) <= 3.402823466e38f) {
+      const float sum = survivor_sum(sorted, kept, n, row.size, mx, false, seg, s_nan), inv = 1.0f / sum;
+      const int bits = mass_bits(n, row.size);
+      const float unit = ldexpf(1.0f, 24 + bits);
+      const unsigned long long target = max((unsigned long long)ceil((double)ch.p * (double)unit), 1ull);
+      unsigned long long* const mass = reinterpret_cast<unsigned long long*>(bins);
+      for (int j = tid; j < kept; j += kThreads) mass[j] = __float2ull_rn(expf(value(j) - mx) * inv * unit);
+      __syncthreads();
+      kept = leading([&](int j) {
+        unsigned long long ahead = 0;
+        for (int i = 0; i < j; ++i) ahead += mass[i];
+        return ahead < target;
+      });
+    }
+    if (ch.min_p > 0.0f && kept) {
+      const float sum = survivor_sum(sorted, kept, n, row.size, mx, false, seg, s_nan);
+      const bool norm = sum > 0.0f;
+      const float threshold = ch.min_p * (norm ? 1.0f / sum : 1.0f);
+      kept = leading([&](int j) {
+        float pr = expf(value(j) - mx);
+        if (norm) pr /= sum;
+        return !(pr < threshold);
+      });
+    }
+    if (ch.uniforms) {
+      const float sum = survivor_sum(sorted, kept, n, row.size, mx, true, seg, s_nan);
+      int2* const by_index = room;  // (index, probability)
+      for (int j = tid; j < kept; j += kThreads) {
+        const int own = sorted[j].x;
+        const float v = value(j);
+        int rank = 0;
+        for (int i = 0; i < kept; ++i) rank += sorted[i].x < own ? 1 : 0;
+        // without mass anywhere the first maximum is taken
+        const float pr = !(sum > 0.0f) ? (v == mx ? 1.0f : 0.0f) : fabsf(v) <= 3.402823466e38f ? expf(v - mx) / sum : 0.0f;
+        by_index[rank] = make_int2(own, __float_as_int(pr));
+      }
+      __syncthreads();
+      if (warp == 0) {
+        const int out_row = blockIdx.x / row.size;
+        float r = sum > 0.0f ? ch.uniforms[out_row] : 0.0f;
+        int token = 0;  // the last value with mass where rounding carries the draw past all of them
+        for (int j0 = 0; j0 < kept; j0 += 32) {
+          const int j = j0 + lane;
+          const float pr = j < kept ? __int_as_float(by_index[j].y) : 0.0f;
+          float incl = pr;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          const uint32_t has = __ballot_sync(0xffffffffu, pr > 0.0f), hit = __ballot_sync(0xffffffffu, pr > 0.0f && r < incl);
+          if (has) token = by_index[j0 + (hit ? __ffs(hit) - 1 : 31 - __clz(has))].x;
+          if (hit) break;
+          r -= __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) ch.out[out_row] = (uint32_t)token;
+      }
+    }
+  }
+  row_sync(c, row);  // the row is -inf
+  if (row.rank == 0)
+    for (int j = tid; j < kept; j += kThreads) row.l[sorted[j].x] = __int_as_float(sorted[j].y);
+}
+
 // a row is a cluster of eight CTAs, or one CTA
 template <typename... P, typename... A>
 uint32_t launch_rows(void (*kern)(P...), int rows, int n, void* stream, A... args) {
@@ -611,6 +858,7 @@ uint32_t logismos_launch_top_k_f32(void* logits, int32_t rows, int32_t n, int32_
   lg::LaunchScope launch_scope_;
   if (rows < 0 || n < 0 || k < 0 || !logits) return lg::kInvalidValue;
   if (k == 0 || k >= n || rows == 0) return 0;
+  if (k <= kFewK) return launch_rows(few_survivors_kernel, rows, n, stream, (float*)logits, n, Chain{1.0f, k, 1.0f, 0.0f, nullptr, nullptr});
   return launch_rows(top_k_kernel, rows, n, stream, (float*)logits, n, k);
 }
 
@@ -647,6 +895,23 @@ uint32_t logismos_launch_multinomial_f32(const void* logits, int32_t rows, int32
   if (rows == 0) return 0;
   if (n == 0) return (uint32_t)cudaMemsetAsync(out_u32, 0, (size_t)rows * 4, (cudaStream_t)stream);  // an empty slice samples 0
   return launch_rows(multinomial_kernel, rows, n, stream, (const float*)logits, n, (const float*)uniforms_f32, (uint32_t*)out_u32);
+}
+
+uint32_t logismos_launch_sample_chain_f32(void* logits, int32_t rows, int32_t n, float temperature, int32_t k, float p, float min_p, const void* uniforms_f32,
+                                          void* out_u32, void* stream) {
+  lg::LaunchScope launch_scope_;
+  if (rows < 0 || n < 0 || k < 0 || !logits || !out_u32 || (rows > 0 && n > 0 && !uniforms_f32)) return lg::kInvalidValue;
+  if (rows == 0) return 0;
+  if (k > 0 && k <= kFewK && k < n) {
+    const float t = fmaxf(temperature, 1e-6f);
+    return launch_rows(few_survivors_kernel, rows, n, stream, (float*)logits, n,
+                       Chain{fabsf(t - 1.0f) < 1e-9f ? 1.0f : t, k, fminf(fmaxf(p, 0.0f), 1.0f), fminf(fmaxf(min_p, 0.0f), 1.0f), (const float*)uniforms_f32, (uint32_t*)out_u32});
+  }
+  uint32_t rc = logismos_launch_temperature_f32(logits, rows, n, temperature, stream);
+  if (!rc) rc = logismos_launch_top_k_f32(logits, rows, n, k, stream);
+  if (!rc) rc = logismos_launch_top_p_f32(logits, rows, n, p, stream);
+  if (!rc) rc = logismos_launch_min_p_f32(logits, rows, n, min_p, stream);
+  return rc ? rc : logismos_launch_multinomial_f32(logits, rows, n, uniforms_f32, out_u32, stream);
 }
 
 }  // extern "C"

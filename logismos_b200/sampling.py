@@ -119,8 +119,12 @@ class MultinomialSampler:
         return out
 
 
+_FUSED = {TemperatureScale: 0, TopK: 1, TopP: 2, MinP: 3}  # the places of a chain that runs as one launch
+
+
 class DecodeChain:
-    """chain.rs:33-76: processors in insertion order, then the sampler."""
+    """chain.rs:33-76: processors in insertion order, then the sampler. Temperature, top-k, top-p and min-p in that order with a
+    multinomial draw run as one launch where k is at most 256, with the same results."""
 
     def __init__(self, sampler):
         self.processors, self.sampler = [], sampler
@@ -129,7 +133,27 @@ class DecodeChain:
         self.processors.append(p)
         return self
 
+    def _settings(self):
+        """(temperature, k, p, min_p) of a chain that is some of these in this order, with a top-k, and a multinomial draw; None for others."""
+        if type(self.sampler) is not MultinomialSampler:
+            return None
+        out, at = [1.0, 0, 1.0, 0.0], -1
+        for q in self.processors:
+            i = _FUSED.get(type(q), -1)
+            if i <= at:
+                return None
+            at = i
+            out[i] = q.t if i == 0 else q.k if i == 1 else q.p
+        return out if out[1] > 0 else None
+
     def step(self, logits, ctx=None):
+        settings = self._settings()
+        if settings is not None:  # one launch
+            r, n = _rows(logits)
+            uniforms = torch.rand(r, generator=self.sampler.gen, device=logits.device, dtype=torch.float32)
+            out = torch.empty(r, dtype=torch.int32, device=logits.device)
+            check(lib.logismos_launch_sample_chain_f32(_p(logits), r, n, *settings, _p(uniforms), _p(out), _stream()), "sample_chain")
+            return out
         for p in self.processors:
             p.process(logits, ctx)
         return self.sampler.sample(logits)

@@ -248,3 +248,56 @@ def test_top_p_of_long_rows_keeps_small_probabilities(n):
         pr = probs64(x)
         m = pr[keep].sum()
         assert p * (1 - 2e-6) <= m <= p * (1 + 2e-6) + pr[keep].min(), (p, m)
+
+
+def _apart(chain, x, u):
+    """The chain's processors one by one and the draw from the uniforms u."""
+    t = torch.from_numpy(x.copy()).to(DEV)
+    for p in chain.processors:
+        p.process(t)
+    return t, S.MultinomialSampler(seed=1).sample(t, uniforms=u)
+
+
+@pytest.mark.parametrize("n", [2, 5, 255, 300, 1500, 2047, 2048, 2050, 8195, 33001, 151936, 262150])
+@pytest.mark.parametrize("k", [1, 2, 50, 256, 257])
+def test_a_chain_in_one_launch_leaves_what_its_processors_leave(n, k):
+    """Temperature, top-k, top-p, min-p and draw as one launch against one launch each: the same survivors to the bit. Rows of random values, of few values (more ties
+    at the cut than the launch lists), of one value, with fewer finite values than k, with NaN and infinities, with the largest values side by side, all -inf; rows that
+    start off a 16-byte boundary (odd n). k below, at and above the largest that the launch takes. Draws may differ where both lie within 1e-5 of the draw
+    in the survivors' cumulative mass (fp32 sums of at most 512 normalised masses in another order)."""
+    rng = np.random.default_rng([n, k])
+    x = (rng.standard_normal((9, n)) * 3.0).astype(np.float32)
+    x[1] = np.round(x[1]) + 0.0
+    x[2] = 0.25
+    x[3, rng.random(n) < 0.995] = -np.inf
+    x[4, :: 3] = np.nan
+    x[5, n // 2] = np.inf
+    x[5, -1] = np.inf
+    x[6] = np.sort(x[6])
+    x[7] = -np.inf
+    x[8] *= 1e-3
+    u = torch.from_numpy(rng.random(9).astype(np.float32)).to(DEV)
+    for t, p, m in ((1.0, 1.0, 0.0), (0.8, 0.95, 0.0), (1.7, 0.3, 0.02), (1e-7, 0.0, 0.5), (0.7, 1.0, 0.1)):
+        chain = S.DecodeChain(S.MultinomialSampler(seed=1)).push(S.TemperatureScale(t)).push(S.TopK(k)).push(S.TopP(p)).push(S.MinP(m))
+        ref, ref_tokens = _apart(chain, x, u)
+        got, tokens = torch.from_numpy(x.copy()).to(DEV), torch.empty(9, dtype=torch.int32, device=DEV)
+        S.check(S.lib.logismos_launch_sample_chain_f32(S._p(got), 9, n, *chain._settings(), S._p(u), S._p(tokens), S._stream()), "sample_chain")
+        assert torch.equal(got.view(torch.int32), ref.view(torch.int32)), (t, p, m, (got.view(torch.int32) != ref.view(torch.int32)).nonzero()[:5])
+        for r in (tokens != ref_tokens).nonzero().flatten().tolist():
+            row = got[r].double().cpu().numpy()
+            cdf, (a, b) = np.cumsum(np.where(np.isfinite(row), probs64(row), 0.0)), sorted((int(tokens[r]), int(ref_tokens[r])))
+            assert np.isfinite(row[a]) and np.isfinite(row[b]) and abs(cdf[a] - float(u[r])) <= 1e-5 and cdf[b - 1] - cdf[a] <= 1e-5, (t, p, m, r)
+        chain.sampler = S.MultinomialSampler(seed=5)
+        stepped = torch.from_numpy(x.copy()).to(DEV)
+        drawn = chain.step(stepped)
+        v = torch.rand(9, generator=S.MultinomialSampler(seed=5).gen, device=DEV, dtype=torch.float32)
+        S.check(S.lib.logismos_launch_sample_chain_f32(S._p(got.copy_(torch.from_numpy(x))), 9, n, *chain._settings(), S._p(v), S._p(tokens), S._stream()), "sample_chain")
+        assert torch.equal(stepped.view(torch.int32), ref.view(torch.int32)) and torch.equal(drawn, tokens)
+
+
+def test_chains_of_another_shape_run_one_launch_per_processor():
+    m = S.MultinomialSampler
+    for chain in (S.DecodeChain(S.GreedySampler()).push(S.TopK(3)), S.DecodeChain(m(1)).push(S.TopP(0.9)), S.DecodeChain(m(1)).push(S.TopK(3)).push(S.TemperatureScale(0.5)),
+                  S.DecodeChain(m(1)).push(S.TopK(3)).push(S.TopK(2)), S.DecodeChain(m(1)).push(S.TopK(-1)), S.DecodeChain(m(1)).push(S.TopK(3)).push(S.TypicalSampling(0.5)), S.DecodeChain(m(1))):
+        assert chain._settings() is None
+    assert S.DecodeChain(m(1)).push(S.TopK(3))._settings() == [1.0, 3, 1.0, 0.0]
