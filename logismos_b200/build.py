@@ -25,7 +25,7 @@ SO = os.path.join(HERE, "liblogismos_kernels.so")
 AR = os.path.join(HERE, "liblogismos_kernels.a")
 
 CU_SOURCES = ["cudacore.cu", "legacy_fp16.cu", "elementwise.cu", "gemv_int4.cu", "int4_rows.cu", "dequant_int4.cu", "gemm_tcgen05.cu", "qgemm_tcgen05.cu",
-              "attention.cu", "attention_tcgen05.cu", "short_attention.cu", "gdn.cu", "gdn_chunk.cu", "sampling.cu", "kvquant.cu", "stella_model.cu", "decoder_model.cu", "hybrid_model.cu", "tp_comm.cu",
+              "attention.cu", "attention_tcgen05.cu", "short_attention.cu", "gdn.cu", "gdn_chunk.cu", "sampling.cu", "kvquant.cu", "decode_stack.cu", "stella_model.cu", "decoder_model.cu", "hybrid_model.cu", "tp_comm.cu",
               "linear_small.cu", "depth_conv.cu", "latent_attention.cu", "latent_model.cu",
               "post_norm.cu", "tanh_norm.cu", "time_mix.cu", "ssd.cu", "bias_attention.cu", "rotary.cu", "moe.cu", "mixer_parallel.cu",
               "gated_residual.cu", "mixer_gated.cu", "mixer_paired.cu", "mixer_model.cu"]

@@ -179,6 +179,19 @@ LG_DEVINL float2 unpack_bf16x2(uint32_t u) {
   return __bfloat1622float2(v);
 }
 
+// (w & mask) ^ flip in one logic operation. The masks come from opaque(): with two constants that the compiler knows it makes two operations of it, of
+// which one can hold an immediate each, and unpacking int4 is bound by these (a warp's 2048 weights: 83 operations on the ALU pipe with them, 56 without).
+LG_DEVINL uint32_t and_xor(uint32_t w, uint32_t mask, uint32_t flip) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0x6a;\n" : "=r"(r) : "r"(w), "r"(mask), "r"(flip));
+  return r;
+}
+LG_DEVINL uint32_t opaque(uint32_t v) {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %1;\n" : "=r"(r) : "r"(v));
+  return r;
+}
+
 // 16-byte async copy global -> shared, bypassing L1 (data is streamed once).
 LG_DEVINL void cp_async16(uint32_t smem_addr, const void* gptr) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr), "l"(gptr));

@@ -1,0 +1,58 @@
+// All layers of a decode step of one to four sequences in one launch, for the int4 decoder (decode_stack.cu).
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace lg {
+
+struct StackMat {
+  const uint8_t* codes;  // [n][k / 2]
+  const __half* scales;  // [n][k / 32]
+};
+struct StackLayer {  // an array of these on the device
+  const float *norm1, *norm2, *bias;  // bias: of q | k | v
+  StackMat qkv, out, gate_up, down;   // gate_up: 32 gate rows, then the 32 matching up rows
+  __nv_bfloat16 *k_pool, *v_pool;
+};
+
+struct StackDims { int hidden, inter, n_heads, n_kv, rows; };  // heads of 128
+
+// How a launch is laid out: what each of the CTAs takes of every matrix, and the shared memory for it.
+struct StackPlan {
+  int ctas, warps;         // a warp per 128 values of the hidden size
+  int qkv_tiles, gu_tiles; // tiles of 16 weight rows (8 pairs) per CTA
+  int out_rows;            // rows of the output and down projections per CTA
+  int att_warps;           // warps of a CTA that take cache blocks
+  int max_chunks;          // chunks of a context at most
+  // offsets of the parts of shared memory: rows of q, k, v | output | gate, up | down and their scales, activations, angles of q, k, v, sums of activations, the warps' sums (part_step bytes each)
+  uint32_t at[4], at_scales[4], at_x, at_turn, at_sums, at_part, part_step, bytes;
+};
+bool stack_plan(const StackDims& d, StackPlan* plan);
+// tokens per chunk of the longest of `rows` contexts
+int stack_chunk(const StackPlan& plan, const int32_t* ctx, int rows);
+// No row's new token goes to a block that another row, or another place of its own table, holds: blocks without a new token may be read before it is stored.
+bool stack_blocks_apart(const int32_t* tables, int max_blocks, const int32_t* ctx, int rows);
+// 64-bit words by which the CTAs of launches of up to d.rows rows pass on results; all zero before the first launch and after a failed one
+size_t stack_words(const StackDims& d);
+
+struct StackArgs {
+  StackDims d;
+  const StackLayer* layers;
+  int n_layers;
+  float eps;
+  float* x;  // [rows][hidden], in place
+  const float *cos, *sin;  // [max_pos][64]
+  const int* positions;
+  int max_pos;
+  const int64_t* slots;
+  const int *ctx, *tables;
+  int max_blocks, n_pool_blocks, chunk;
+  unsigned long long* words;  // stack_words
+  uint32_t* launches;         // how many went before, with the words
+  int* status;
+};
+uint32_t launch_decode_stack(const StackArgs& a, const StackPlan& plan, cudaStream_t stream);
+
+}  // namespace lg

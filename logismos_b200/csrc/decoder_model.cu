@@ -13,6 +13,7 @@
 //   tables, so a chunk may continue a cached sequence) -> o_proj + residual ->
 //   rms_norm -> gate/up with SwiGLU fused in the GEMM epilogue -> down + residual ] -> last token rows -> final norm ->
 //   lm_head (int4 GEMV) -> greedy argmax.
+// A pure decode step of up to four sequences runs its layers as one launch (decode_stack.cu) where the widths fit it.
 // Contractions over the packed rows run on the tcgen05 GEMM over a per-layer bf16 expansion of the
 // int4 codes; the lm_head, whose batch is the number of sequences, runs on the int4 GEMV kernel.
 #include <cuda_runtime.h>
@@ -27,6 +28,7 @@
 #include "logismos_kernels.h"
 #include "logismos_model.h"
 
+#include "decode_stack.h"
 #include "model_util.h"
 #include "step_batch.h"
 
@@ -51,12 +53,14 @@ struct Decoder {
   // workspace
   Buf x, h, qkv, attn, qdec, gu, act, wscratch, accws, last, last_bf16, logits, tokens, status;
   Buf ids, pos, slots, cu_prefill, last_idx, dec_ctx, dec_tables, dec_chunks, dec_scratch, attn_ws, pre_kv;
+  Buf stack_layers, stack_words;  // of decode_stack.cu
+  bool stack = false;             // the device launches grids whose CTAs wait for one another
   HostRows host_rows;
   StepBatch batch;  // the last step (kept for replay and diagnostics)
   cudaStream_t stream = nullptr;
   std::mutex mu;
   int T = 0, n_dec = 0, n_pre = 0, n_seqs = 0, max_pre_len = 0, total_chunks = 0, chunk_tokens = kChunkTokens, launches = 0, logits_f32 = 0;
-  size_t max_chunks = 0;
+  size_t max_chunks = 0, stack_words_bytes = 0;
   // the fused int4 linears rely on `accws` being all zero between calls, which their finishing kernels
   // restore; a step that failed part-way may have left partial sums there, so the next one clears it
   bool acc_dirty = false;
@@ -77,13 +81,29 @@ uint32_t run_device(Decoder* m, cudaStream_t s) {
   m->launches = 0;
   if (m->acc_dirty) {
     LG_TRY(cudaMemsetAsync(m->accws.p, 0, m->accws_bytes, s), "clear accumulation workspace");
+    LG_TRY(cudaMemsetAsync(m->stack_words.p, 0, m->stack_words_bytes, s), "clear words");
     m->acc_dirty = false;
   }
   LG_TRY(logismos_launch_embed_lookup_bf16(m->tok_embed.p, m->ids.p, m->x.p, T, H, c.vocab, s), "embed_lookup");
   m->launches += 1;
   // not under the deterministic switch: a row's bits must not depend on how many share its step
   const bool few = !logismos_get_deterministic() && m->n_pre == 0 && lg::int4_rows_fit(T, std::max(H, I)) && !c.kv_turbo3;
-  for (int l = 0; l < c.n_layers; ++l) {
+  const lg::StackDims dims{H, I, c.n_heads, c.n_kv_heads, T};
+  lg::StackPlan plan;
+  const bool stack = few && m->stack && lg::stack_plan(dims, &plan) && lg::stack_blocks_apart(m->batch.tables, c.max_blocks_per_seq, m->batch.ctx, T);
+  if (stack) {
+    lg::StackArgs a{};
+    a.d = dims;
+    a.layers = (const lg::StackLayer*)m->stack_layers.p; a.n_layers = c.n_layers; a.eps = c.rms_eps;
+    a.x = (float*)m->x.p;
+    a.cos = (const float*)m->cos.p; a.sin = (const float*)m->sin.p; a.positions = (const int*)m->pos.p; a.max_pos = c.max_pos; a.slots = (const int64_t*)m->slots.p;
+    a.ctx = (const int*)m->dec_ctx.p; a.tables = (const int*)m->dec_tables.p; a.max_blocks = c.max_blocks_per_seq; a.n_pool_blocks = c.n_pool_blocks;
+    a.chunk = lg::stack_chunk(plan, m->batch.ctx, T);
+    a.words = (unsigned long long*)m->stack_words.p; a.launches = (uint32_t*)(a.words + lg::stack_words({H, I, c.n_heads, c.n_kv_heads, lg::kFewRows})); a.status = (int*)st;
+    LG_TRY(lg::launch_decode_stack(a, plan, s), "layers of a decode step of few rows");
+    m->launches += 1;
+  }
+  for (int l = 0; l < c.n_layers && !stack; ++l) {
     DLayer& L = m->layers[l];
     if (few) {
       const lg::DecodeHeads heads{D, c.n_heads, c.n_kv_heads, c.max_pos, (const float*)m->cos.p, (const float*)m->sin.p, (const int*)m->pos.p, (const int64_t*)m->slots.p,
@@ -244,7 +264,21 @@ uint32_t lg_decoder_create(int32_t device, const lg_decoder_config_t* cfg, const
        m->tokens.alloc(S * 4) && m->status.alloc(4) && m->ids.alloc(T * 4) && m->pos.alloc(T * 4) && m->slots.alloc(T * 8) &&
        m->cu_prefill.alloc((S + 1) * 4) && m->last_idx.alloc(S * 4) && m->dec_ctx.alloc(S * 4) && m->dec_tables.alloc(S * MB * 4) &&
        m->dec_chunks.alloc((S + 1) * 4) && m->pre_kv.alloc(S * 4) &&
-       m->dec_scratch.alloc(logismos_paged_decode_scratch_bytes((int32_t)m->max_chunks, c.n_heads, m->head_dim));
+       m->dec_scratch.alloc(logismos_paged_decode_scratch_bytes((int32_t)m->max_chunks, c.n_heads, m->head_dim)) &&
+       m->stack_words.alloc(m->stack_words_bytes = 8 * (1 + lg::stack_words({(int)H, (int)I, c.n_heads, c.n_kv_heads, lg::kFewRows})));
+  ok = ok && cudaMemset(m->stack_words.p, 0, m->stack_words_bytes) == cudaSuccess;
+  if (ok) {
+    std::vector<lg::StackLayer> t((size_t)c.n_layers);
+    auto mat = [](const QMat& q) { return lg::StackMat{(const uint8_t*)q.codes.p, (const __half*)q.scales.p}; };
+    for (int l = 0; l < c.n_layers; ++l) {
+      const DLayer& L = m->layers[l];
+      t[(size_t)l] = {(const float*)L.norm1.p, (const float*)L.norm2.p, (const float*)L.bqkv.p, mat(L.wqkv), mat(L.wo), mat(L.wgu), mat(L.wdown),
+                      (__nv_bfloat16*)L.kpool.p, (__nv_bfloat16*)L.vpool.p};
+    }
+    int coop = 0;
+    m->stack = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop;
+    ok = m->stack_layers.upload(t.data(), t.size() * sizeof(lg::StackLayer));
+  }
   {
     // the attention workspace serves both prefill routes; the gather route holds one run of sequences at
     // a time, and any single sequence (at most a full block table) must fit
@@ -282,7 +316,8 @@ void lg_decoder_destroy(void* model) {
   cudaSetDevice(m->device);
   Buf* bufs[] = {&m->tok_embed, &m->final_norm, &m->cos, &m->sin, &m->lm_head.codes, &m->lm_head.scales, &m->x, &m->h, &m->qkv,
                  &m->attn, &m->qdec, &m->gu, &m->act, &m->wscratch, &m->accws, &m->last, &m->last_bf16, &m->logits, &m->tokens, &m->status,
-                 &m->ids, &m->pos, &m->slots, &m->cu_prefill, &m->last_idx, &m->dec_ctx, &m->dec_tables, &m->dec_chunks, &m->dec_scratch, &m->attn_ws, &m->pre_kv};
+                 &m->ids, &m->pos, &m->slots, &m->cu_prefill, &m->last_idx, &m->dec_ctx, &m->dec_tables, &m->dec_chunks, &m->dec_scratch, &m->attn_ws, &m->pre_kv,
+                 &m->stack_layers, &m->stack_words};
   for (Buf* b : bufs) b->release();
   for (auto& L : m->layers) {
     Buf* lb[] = {&L.norm1, &L.norm2, &L.bqkv, &L.kpool, &L.vpool, &L.wqkv.codes, &L.wqkv.scales, &L.wo.codes, &L.wo.scales,

@@ -1,4 +1,5 @@
-// int4 group-32 projections of one to four rows, for decode steps of that many sequences.
+// int4 group-32 projections of one to four rows, for decode steps of that many sequences: the hybrid decoder's, and the decoder's at widths that
+// decode_stack.cu does not take.
 //
 // What bounds them is not the 1 to 16 MB of a matrix (0.2 to 2.4 us from HBM) but the length of a launch: start, dependency,
 // one round of latency to memory, a warp's own chain of instructions, the sum over k. The fused-dequant tcgen05 kernel takes 7.6 us
@@ -166,6 +167,7 @@ int4_rows_kernel(const Params p) {
   }
   __syncthreads();
 
+  const uint32_t mask = opaque(0x000f000fu), flip = opaque(0x43084308u);
   const bool col = g < p.rows;  // the activation row of this lane's B values
   const __nv_bfloat16* xg = xs + (size_t)(col ? g : 0) * ld + 8 * t;
   for (int set = blockIdx.x; set < n_sets; set += gridDim.x) {
@@ -181,7 +183,7 @@ int4_rows_kernel(const Params p) {
         transpose4(lo[i], t);
         transpose4(hi[i], t);
         const uint32_t wl[4] = {lo[i].x, lo[i].y, lo[i].z, lo[i].w}, wh[4] = {hi[i].x, hi[i].y, hi[i].z, hi[i].w};
-        auto pair = [](uint32_t w, int n) { return ((w >> (4 * n)) & 0x000f000fu) ^ 0x43084308u; };  // nibbles n, n + 4 as 136 + q
+        auto pair = [=](uint32_t w, int n) { return and_xor(w >> (4 * n), mask, flip); };  // nibbles n, n + 4 as 136 + q
         uint4 x[4];
         float d[4][4];
 #pragma unroll

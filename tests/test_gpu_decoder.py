@@ -154,6 +154,66 @@ def test_decode_steps_of_few_sequences(n_seqs):
     model.close()
 
 
+@pytest.mark.parametrize("heads,kv,inter", [(2, 1, 256), (6, 3, 1280), (8, 1, 512), (12, 1, 512), (16, 2, 2048), (12, 2, 8960)])
+@pytest.mark.parametrize("n_seqs", [1, 2, 3, 4])
+def test_decode_steps_whose_layers_are_one_launch(heads, kv, inter, n_seqs):
+    """Widths at which the layers of a decode step of up to four rows run as one launch (and two, of 16 heads and of 12 to a key head, at which they do not): two to twelve warps,
+    CTAs without a share of a matrix, shares that end in part of a tile, one to eight tiles a CTA, groups of 2 to 8 query heads. Contexts that
+    end a cache block, begin one, are one token and need further rounds of blocks; 3 layers, so that every place in shared memory is filled
+    again and the parity of its barrier comes back."""
+    cfg = dict(TINY, hidden=128 * heads, n_heads=heads, n_kv_heads=kv, intermediate=inter, vocab=520, n_layers=3, max_pos=2048)
+    qw, deq = quantize_weights(cfg, make_weights(cfg, 31))
+    oracle = O.OracleStella(cfg, deq)
+    rng = np.random.default_rng([n_seqs, heads])
+    alloc = BlockAllocator(300, 100, seed=3)
+    model = DecoderModel(cfg, qw, n_pool_blocks=300, max_blocks_per_seq=100, max_step_tokens=1024, max_step_seqs=4)
+    lens = [(130, 1, 47, 16), (15, 700, 30, 1), (1, 31, 128, 97), (250, 16, 3, 5)][n_seqs - 1][:n_seqs]
+    hist = [rng.integers(0, cfg["vocab"], n).tolist() for n in lens]
+    step = lambda ids, cached, new: model.step(ids, cached, new, np.stack([alloc.ensure(i, c + n) for i, (c, n) in enumerate(zip(cached, new))]))
+    for i in range(n_seqs):  # a sequence at a time, so that one of a single token is a decode step as well
+        model.step(hist[i], [0], [lens[i]], alloc.ensure(i, lens[i])[None])
+    for _ in range(5):
+        for h in hist:
+            h.append(int(rng.integers(0, cfg["vocab"])))
+        toks = step([h[-1] for h in hist], [len(h) - 1 for h in hist], [1] * n_seqs)
+        assert model.device_status() == 0 and (model.launches_last_step() <= 7) == (heads <= 12 and heads // kv <= 8)
+    hs, lg = model.last_hidden(), model.last_logits()
+    again = step([h[-1] for h in hist], [len(h) - 1 for h in hist], [1] * n_seqs)
+    assert np.array_equal(hs, model.last_hidden()) and np.array_equal(lg, model.last_logits()) and np.array_equal(toks, again)
+    for i, ids in enumerate(hist):
+        h_ref = oracle.forward(np.asarray(ids, np.uint32), causal=True)[-1]
+        assert max_rel(hs[i], h_ref) <= TOL and max_rel(lg[i], O.linear_t(h_ref, deq["lm_head"], None, 1, cfg["vocab"], cfg["hidden"])) <= TOL, i
+        assert toks[i] == O.greedy(lg[i])
+    model.close()
+
+
+def test_one_launch_and_one_per_projection_on_long_contexts():
+    """Contexts of up to 3000 tokens (several rounds of cache blocks per warp): the layers as one launch against the general route of the
+    deterministic switch. Bound: as the tests against the oracle. Two sequences whose tables share the block of a new token do not take the one launch, which reads blocks
+    ahead of the stores into them."""
+    from logismos_b200._lib import lib
+    cfg = dict(TINY, hidden=768, n_heads=6, n_kv_heads=2, intermediate=1024, vocab=512, max_pos=4096)
+    qw, _ = quantize_weights(cfg, make_weights(cfg, 5))
+    model = DecoderModel(cfg, qw, n_pool_blocks=512, max_blocks_per_seq=200, max_step_tokens=3072, max_step_seqs=4)
+    rng, alloc = np.random.default_rng(1), BlockAllocator(512, 200, seed=2)
+    lens = [3000, 1537, 512]
+    tables = np.stack([alloc.ensure(i, n + 1) for i, n in enumerate(lens)])
+    for i, n in enumerate(lens):
+        model.step(rng.integers(0, 512, n), [0], [n], tables[i:i + 1])
+    out = []
+    for det in (0, 1):
+        lib.logismos_set_deterministic(det)
+        try:
+            model.step([5, 6, 7], lens, [1] * 3, tables)
+            out.append((model.last_hidden().copy(), model.last_logits().copy(), model.launches_last_step()))
+        finally:
+            lib.logismos_set_deterministic(0)
+    assert out[0][2] < out[1][2] and max_rel(out[0][0], out[1][0]) <= TOL and max_rel(out[0][1], out[1][1]) <= TOL
+    model.step([5, 5], [3000, 3000], [1, 1], tables[[0, 0]])
+    assert model.launches_last_step() > 7 and max_rel(model.last_hidden(), out[1][0][[0, 0]]) <= TOL
+    model.close()
+
+
 def test_deterministic_switch_keeps_a_row_independent_of_its_step():
     """With the switch on, a sequence's decode steps have the same bits alone and beside 3, 4 and 29 others: the same projections and the
     same pieces of its context of 1000 tokens."""
