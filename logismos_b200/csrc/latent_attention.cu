@@ -176,7 +176,9 @@ __host__ __device__ constexpr size_t decode_fixed_smem(int rank) {
 }
 
 // MAXKS >= rank / 64: k16 steps of one rank quarter; also the 64-column slabs
-template <int MT, int MAXKS, int TK, bool QREG>
+// EXACT: rank = 64 MAXKS, known to the compiler, which then works out the addresses of shared memory (64 sequences of 2049 tokens, 16 heads, rank 512: 55 us with
+// them worked out per instruction, 39 without; its copies alone take 30, its products alone 32)
+template <int MT, int MAXKS, int TK, bool QREG, bool EXACT>
 __global__ void __launch_bounds__(kDecodeThreads, MT == 1 && MAXKS <= 8 ? 2 : 1)
 latent_decode_kernel(const __grid_constant__ CUtensorMap map_pool, DecodeArgs p, int stages) {
   lg::pdl_trigger();
@@ -185,7 +187,7 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map_pool, DecodeArgs p,
   constexpr int MAXU = (MAXKS * 4 + kWarps - 1) / kWarps;     // 16-column units of the rank per warp
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-  const int R = p.rank, slabs = R >> 6, tile_bytes = TK * R * 2;
+  const int R = EXACT ? 64 * MAXKS : p.rank, slabs = R >> 6, tile_bytes = TK * R * 2;
   uint8_t* after = gen + (size_t)stages * tile_bytes;
   const uint32_t sq = smem_u32(after);                        // [kRows][R] swizzled, when !QREG
   float* s_part = reinterpret_cast<float*>(after + (QREG ? 0 : (size_t)kRows * R * 2));  // [4][kRows][TK + 8]
@@ -282,7 +284,7 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map_pool, DecodeArgs p,
           }
         }
     }
-    const int units = slabs * 4, u_per = (units + kWarps - 1) / kWarps, u0 = warp * u_per, u_n = max(0, min(units - u0, u_per));
+    const int units = slabs * 4, u_per = (units + kWarps - 1) / kWarps, u0 = warp * u_per, u_n = EXACT && MAXKS % 2 == 0 ? u_per : max(0, min(units - u0, u_per));
     float acc[MT][2 * MAXU][4];
 #pragma unroll
     for (int i = 0; i < MT; ++i)
@@ -615,7 +617,7 @@ uint32_t logismos_launch_latent_gather_bf16(const void* pool, const void* block_
 // Chunk length by an estimate in token times: full chunks run in waves over the CTA slots (one CTA per SM, two with few
 // heads), the remainders of the contexts fit the last wave's idle slots or take further waves; a chunk costs a start and a merge share.
 int32_t logismos_pick_latent_chunk(const int32_t* context_lens, int32_t n_seqs, int32_t heads) {
-  static const int32_t cands[] = {128, 192, 256, 320, 384, 448, 512, 640, 768, 896, 1024, 1280, 1536, 1792, 2048, 3072, 4096, 8192, 16384, 1 << 20};
+  static const int32_t cands[] = {128, 192, 256, 320, 384, 448, 512, 576, 640, 704, 768, 832, 896, 960, 1024, 1280, 1536, 1792, 2048, 3072, 4096, 8192, 16384, 1 << 20};
   const int64_t groups = (heads + 63) / 64, slots = heads <= 16 ? 296 : 148, start = 96;
   int32_t best = 0;
   int64_t best_cost = 0;
@@ -672,7 +674,7 @@ uint32_t logismos_launch_latent_decode_bf16(const void* q, const void* pool, con
     return lg::launch_status();
   };
   uint32_t rc;
-#define LG_DECODE(MT, KS, TK, QREG) go(latent_decode_kernel<MT, KS, TK, QREG>, MT, TK, decode_fixed_smem<MT, TK, QREG>(rank), MT == 1 && KS <= 8 ? 2 : 1)
+#define LG_DECODE(MT, KS, TK, QREG) go(rank == 64 * KS ? latent_decode_kernel<MT, KS, TK, QREG, true> : latent_decode_kernel<MT, KS, TK, QREG, false>, MT, TK, decode_fixed_smem<MT, TK, QREG>(rank), MT == 1 && KS <= 8 ? 2 : 1)
   if (rank <= 128) rc = heads <= 16 ? LG_DECODE(1, 2, 64, true) : heads <= 32 ? LG_DECODE(2, 2, 64, true) : LG_DECODE(4, 2, 64, true);
   else if (rank <= 256) rc = heads <= 16 ? LG_DECODE(1, 4, 64, true) : heads <= 32 ? LG_DECODE(2, 4, 64, true) : LG_DECODE(4, 4, 64, true);
   else if (rank <= 512) rc = heads <= 16 ? LG_DECODE(1, 8, 32, true) : heads <= 32 ? LG_DECODE(2, 8, 64, true) : LG_DECODE(4, 8, 32, false);
