@@ -512,35 +512,42 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   if (warp == 0) {
     // ---------------- TMA producer: K(j) as soon as S(j-1) has read its slot, V(j) once PV(j-1) has ----------------
-    if (lane == 0) {
+    // (whole warps go through these loops and one lane issues, see elect_one)
+    if (elect_one()) {
       mbar_expect_tx(q_full, (uint32_t)kQBytes);
 #pragma unroll
       for (int i = 0; i < HD / 64; ++i) tma_load_2d(q_smem + i * kTileBytes, &map_q, q_full, h * HD + i * 64, t0 + q0);
-      const int pv = pstart[s];
-      for (int j = 0; j < nb; ++j) {
-        const uint32_t phase = (uint32_t)j & 1u;
-        const int jt = SCORE == kWindowed && j >= kept ? j + skip : j;
-        if (!mbar_wait(k_empty, phase ^ 1u, abort_flag)) break;
+    }
+    const int pv = pstart[s];
+    for (int j = 0; j < nb; ++j) {
+      const uint32_t phase = (uint32_t)j & 1u;
+      const int jt = SCORE == kWindowed && j >= kept ? j + skip : j;
+      if (!mbar_wait_warp(k_empty, phase ^ 1u, abort_flag)) break;
+      if (elect_one()) {
         mbar_expect_tx(k_full, (uint32_t)kKBytes);
 #pragma unroll
         for (int i = 0; i < HD / 64; ++i) tma_load_2d(k_smem + i * kTileBytes, &map_k, k_full, k_off + kvh * HD + i * 64, k_row0 + jt * 128);
-        if (!mbar_wait(v_empty, phase ^ 1u, abort_flag)) break;
+      }
+      __syncwarp();
+      if (!mbar_wait_warp(v_empty, phase ^ 1u, abort_flag)) break;
+      if (elect_one()) {
         mbar_expect_tx(v_full, (uint32_t)kVBytes);
         tma_load_2d(v_smem, &map_vt, v_full, pv + jt * 128, kvh * HD);
         tma_load_2d(v_smem + kVTile, &map_vt, v_full, pv + jt * 128 + 64, kvh * HD);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     // The tensor pipe runs the MMAs of one CTA in issue order, so S(j) (issued after PV(j-1)) never
     // overwrites the P columns PV(j-1) still reads, and "S(j) complete" implies "PV(j-1) complete".
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc<128>(), idesc_o = make_idesc<HD>();
-      bool ok = mbar_wait(q_full, 0u, abort_flag);
-      for (int j = 0; j < nb && ok; ++j) {
-        const uint32_t phase = (uint32_t)j & 1u;
-        if (!mbar_wait(k_full, phase, abort_flag)) { ok = false; break; }
-        tc_fence_after();
+    constexpr uint32_t idesc_s = make_idesc<128>(), idesc_o = make_idesc<HD>();
+    bool ok = mbar_wait_warp(q_full, 0u, abort_flag);
+    for (int j = 0; j < nb && ok; ++j) {
+      const uint32_t phase = (uint32_t)j & 1u;
+      if (!mbar_wait_warp(k_full, phase, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
           const uint64_t da = make_smem_desc(q_smem + (kk >> 2) * kTileBytes) + (uint64_t)(2 * (kk & 3));
@@ -549,9 +556,12 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         tc_commit(s_full);
         tc_commit(k_empty);
-        if (!mbar_wait(p_full, phase, abort_flag)) { ok = false; break; }
-        if (!mbar_wait(v_full, phase, abort_flag)) { ok = false; break; }
-        tc_fence_after();
+      }
+      __syncwarp();
+      if (!mbar_wait_warp(p_full, phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(v_full, phase, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint64_t db = make_smem_desc(v_smem + (kk >> 2) * kVTile) + (uint64_t)(2 * (kk & 3));
@@ -560,6 +570,7 @@ attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_commit(v_empty);
         if (j == nb - 1) tc_commit(o_done);
       }
+      __syncwarp();
     }
   } else {
     // ---------------- softmax and epilogue: thread = query row ----------------
