@@ -498,6 +498,168 @@ gdn_decode_fused_kernel(float* __restrict__ state, float* __restrict__ acc, int6
   }
 }
 
+// The same step for batches whose halves of heads do not all fit at once. What bounds it is the 128 KB of state per (sequence, head) that cross HBM; the
+// kernel above leaves a part of that rate unused, since its CTAs load, compute and store in step and the last of its 3.5 waves (64 sequences of 16 heads) is half
+// empty. Here a CTA holds one whole head's state in shared memory (64 KB, three CTAs per SM, so 192 KB of reads in flight) and walks over several heads: every
+// thread copies, uses and writes back only its own 32 rows x 4 columns, so the copies of the next head start row by row behind the last use of this one and need no
+// barrier, and the vectors of the next head are read while this one is computed. Each partial sum covers the same rows in the same order as above: the same bits.
+// One CTA per head also means that nobody else reads its columns of the workspace, so there is no counter.
+__global__ void __launch_bounds__(128, 3)
+gdn_decode_walk_kernel(float* __restrict__ state, float* __restrict__ acc, int64_t ld_acc, const float* __restrict__ A_log,
+                       const float* __restrict__ dt_bias, __nv_bfloat16* __restrict__ o, const int* __restrict__ slots,
+                       const uint8_t* __restrict__ fresh, int heads, int items, float scale) {
+  lg::pdl_trigger();
+  constexpr int KS = 4, R = KD / KS;
+  extern __shared__ __align__(16) float4 own_s[];  // [R][128 threads]
+  __shared__ __align__(16) float vec_s[2][4][KD];  // q, k, v, z of this head and the one before
+  __shared__ float gate_s[2][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kq = lane >> 3, col = warp * 32 + (lane & 7) * 4;  // eight lanes read 128 bytes of a row
+  float4* own = own_s + tid;
+  const uint32_t own_a = smem_u32(own);
+  auto state_of = [&](int it) {
+    const int seq = it / heads;
+    const int64_t slot = slots ? slots[seq] : seq;
+    return state + (slot * heads + it % heads) * (int64_t)(KD * VD) + (kq * R) * VD + col;
+  };
+  auto fetch_row = [&](const float* src, bool zero, int i) {
+    if (zero) own[i * 128] = make_float4(0.f, 0.f, 0.f, 0.f);
+    else cp_async16(own_a + i * 128 * 16, src + i * VD);
+  };
+  int it = blockIdx.x;
+  float* hp = state_of(it);
+  {
+    const bool zero = fresh && fresh[it / heads];
+#pragma unroll 8
+    for (int i = 0; i < R; ++i) fetch_row(hp, zero, i);
+    cp_async_commit();
+  }
+  lg::pdl_wait();
+  const int w = heads * KD;
+  float4 x;
+  float ga = 0.f, gb = 0.f;
+  // takes the warp's vector (and the gates' inputs) of a head out of the workspace, which is left zeroed for the next accumulation
+  auto take = [&](int n) {
+    const int head = n % heads;
+    float* arow = acc + (int64_t)(n / heads) * ld_acc;
+    float4* src = reinterpret_cast<float4*>(arow + warp * w + head * KD + lane * 4);
+    x = *src;
+    *src = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tid == 96) {
+      float* ab = arow + 4 * w + head;
+      ga = ab[0];
+      gb = ab[heads];
+      ab[0] = 0.f;
+      ab[heads] = 0.f;
+    }
+  };
+  take(it);
+#pragma unroll 1
+  for (int buf = 0;; buf ^= 1) {
+    const int head = it % heads;
+    if (warp < 2) {  // q and k: unit L2 norm in fp32
+      const float sq = warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w);
+      const float inv = 1.0f / fmaxf(sqrtf(sq), 1e-12f);
+      x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
+    }
+    const float2 lo = unpack_bf16x2(pack_bf16x2(x.x, x.y)), hi = unpack_bf16x2(pack_bf16x2(x.z, x.w));  // one bf16 rounding
+    *reinterpret_cast<float4*>(&vec_s[buf][warp][lane * 4]) = make_float4(lo.x, lo.y, hi.x, hi.y);
+    if (tid == 96) {
+      const float a = ga + dt_bias[head];
+      const float sp = a > 20.0f ? a : log1pf(expf(a));
+      gate_s[buf][0] = -expf(A_log[head]) * sp;
+      gate_s[buf][1] = 1.0f / (1.0f + expf(-gb));
+    }
+    __syncthreads();  // the only one per head: the buffers alternate
+    const int nx = it + gridDim.x;
+    const bool more = nx < items;
+    const float* np = nullptr;
+    bool nzero = false;
+    if (more) {
+      take(nx);
+      np = state_of(nx);
+      nzero = fresh && fresh[nx / heads];
+    }
+    const float decay = expf(gate_s[buf][0]);
+    const float b_cur = gate_s[buf][1];
+    const float4 vv = *reinterpret_cast<const float4*>(&vec_s[buf][2][col]), zz = *reinterpret_cast<const float4*>(&vec_s[buf][3][col]);
+    const float v_cur[4] = {vv.x, vv.y, vv.z, vv.w}, z_cur[4] = {zz.x, zz.y, zz.z, zz.w};
+    const float4* q4 = reinterpret_cast<const float4*>(&vec_s[buf][0][kq * R]);
+    const float4* k4 = reinterpret_cast<const float4*>(&vec_s[buf][1][kq * R]);
+    float a4[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) a4[a][cc] = 0.f;
+    cp_async_wait<0>();
+#pragma unroll 4
+    for (int j = 0; j < R / 4; ++j) {
+      const float4 kv = k4[j];
+      const float kk[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const float4 h = own[(4 * j + a) * 128];
+        a4[a][0] += h.x * kk[a];
+        a4[a][1] += h.y * kk[a];
+        a4[a][2] += h.z * kk[a];
+        a4[a][3] += h.w * kk[a];
+      }
+    }
+    float vd[4];
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
+      float hk = (a4[0][cc] + a4[1][cc]) + (a4[2][cc] + a4[3][cc]);
+      hk += __shfl_xor_sync(0xffffffffu, hk, 8);
+      hk += __shfl_xor_sync(0xffffffffu, hk, 16);
+      vd[cc] = b_cur * (v_cur[cc] - decay * hk);
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) a4[a][cc] = 0.f;
+#pragma unroll 4
+    for (int j = 0; j < R / 4; ++j) {
+      const float4 kv = k4[j], qv = q4[j];
+      const float kk[4] = {kv.x, kv.y, kv.z, kv.w}, qq[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        float4 h = own[(4 * j + a) * 128];
+        h.x = fmaf(h.x, decay, kk[a] * vd[0]);
+        h.y = fmaf(h.y, decay, kk[a] * vd[1]);
+        h.z = fmaf(h.z, decay, kk[a] * vd[2]);
+        h.w = fmaf(h.w, decay, kk[a] * vd[3]);
+        *reinterpret_cast<float4*>(hp + (4 * j + a) * VD) = h;
+        a4[a][0] += h.x * qq[a];
+        a4[a][1] += h.y * qq[a];
+        a4[a][2] += h.z * qq[a];
+        a4[a][3] += h.w * qq[a];
+      }
+      if (more) {  // these rows have been used: the next head's take their place
+#pragma unroll
+        for (int a = 0; a < 4; ++a) fetch_row(np, nzero, 4 * j + a);
+      }
+    }
+    cp_async_commit();
+    float ov[4];
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
+      float s = (a4[0][cc] + a4[1][cc]) + (a4[2][cc] + a4[3][cc]);
+      s += __shfl_xor_sync(0xffffffffu, s, 8);
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
+      s *= scale;
+      ov[cc] = s * (z_cur[cc] / (1.0f + __expf(-z_cur[cc])));
+    }
+    if (kq == 0) {
+      __nv_bfloat16* dst = o + (int64_t)it * VD + col;
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) dst[cc] = __float2bfloat16(ov[cc]);
+    }
+    if (!more) break;
+    it = nx;
+    hp = const_cast<float*>(np);
+  }
+}
+
 }  // namespace
 
 extern "C" uint32_t logismos_launch_gdn_finish(void* acc, int32_t ld_acc, const void* A_log, const void* dt_bias, void* proj,
@@ -526,6 +688,16 @@ extern "C" uint32_t logismos_launch_gdn_decode_from_acc(void* state, void* acc, 
   if (((uintptr_t)state & 15) || ((uintptr_t)acc & 15) || ((uintptr_t)o & 1) || ((uintptr_t)pair_count & 3)) return lg::kInvalidValue;
   const int64_t ctas = (int64_t)n_seqs * heads * PfCfg<2, 4>::kParts;
   if (ctas > 2147483647ll) return lg::kInvalidValue;
+  if (ctas > 4ll * lg::sm_count()) {  // more than the kernel of halves holds at once
+    constexpr size_t smem = (size_t)KD * VD * 4;
+    const cudaError_t e = lg::allow_shared((const void*)gdn_decode_walk_kernel, smem);
+    if (e != cudaSuccess) return (uint32_t)e;
+    const int items = n_seqs * heads, grid = items < 3 * lg::sm_count() ? items : 3 * lg::sm_count();
+    lg::launch(gdn_decode_walk_kernel, dim3((unsigned)grid), dim3(128), smem, (cudaStream_t)stream, (float*)state, (float*)acc,
+               (int64_t)ld_acc, (const float*)A_log, (const float*)dt_bias, (__nv_bfloat16*)o, (const int*)state_slots,
+               (const uint8_t*)fresh, heads, items, scale);
+    return lg::launch_status();
+  }
   lg::launch(gdn_decode_fused_kernel, dim3((unsigned)ctas), dim3(128), 0, (cudaStream_t)stream, (float*)state, (float*)acc,
              (int64_t)ld_acc, (const float*)A_log, (const float*)dt_bias, (__nv_bfloat16*)o, (const int*)state_slots,
              (const uint8_t*)fresh, (int*)pair_count, heads, scale);

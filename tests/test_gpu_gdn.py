@@ -160,6 +160,36 @@ def test_decode_from_the_workspace_equals_finish_then_recurrence():
     assert np.isfinite(to_np(o_b)).all()
 
 
+@pytest.mark.parametrize("T,heads", [(50, 6), (61, 8), (64, 16)])
+def test_decode_of_a_large_batch_equals_decode_in_parts(T, heads):
+    """Batches whose CTAs walk over several heads (one, two and three heads per CTA) against the same sequences in calls small enough for one half of a head per CTA: outputs, states and the
+    zeroed workspace bit for bit; state slots permuted, fresh sequences first, last and between."""
+    from logismos_b200._lib import check, lib
+    rng = np.random.default_rng(T)
+    D = 128
+    W = heads * D
+    ld = 4 * W + 2 * heads
+    acc0 = torch.from_numpy(rng.standard_normal((T, ld)).astype(np.float32)).to(DEV)
+    A_t = torch.from_numpy(rng.uniform(-1, 0.5, heads).astype(np.float32)).to(DEV)
+    dt_t = torch.from_numpy(rng.standard_normal(heads).astype(np.float32)).to(DEV)
+    state0 = torch.from_numpy((rng.standard_normal((T + 3, heads, D, D)) * 0.05).astype(np.float32)).to(DEV)
+    slots = torch.from_numpy(rng.permutation(T + 3)[:T].astype(np.int32)).to(DEV)
+    fresh = torch.zeros(T, dtype=torch.uint8, device=DEV)
+    fresh[[0, T // 2, T - 1]] = 1
+
+    def run(part):
+        acc, st, o = acc0.clone(), state0.clone(), torch.empty((T, W), dtype=torch.bfloat16, device=DEV)
+        pairs = torch.zeros(T * heads, dtype=torch.int32, device=DEV)
+        for t in range(0, T, part):
+            check(lib.logismos_launch_gdn_decode_from_acc(st.data_ptr(), acc[t:].data_ptr(), ld, A_t.data_ptr(), dt_t.data_ptr(), o[t:].data_ptr(), slots[t:].data_ptr(),
+                                                          fresh[t:].data_ptr(), pairs.data_ptr(), min(part, T - t), heads, D ** -0.5, torch.cuda.current_stream().cuda_stream), "decode")
+        torch.cuda.synchronize()
+        return o, st, acc, pairs
+
+    for got, want in zip(run(T), run(8)):
+        assert torch.equal(got, want) and bool(torch.isfinite(got.float()).all())
+
+
 def test_both_kernel_shapes_agree_with_the_reference():
     """The throughput shape (64 columns per CTA, key rows in quarters) and the latency shape (32 columns, one per thread) against the oracle's recurrence, from a non-zero state, ragged lengths that
     end inside and on the eight-token staging chunks."""
