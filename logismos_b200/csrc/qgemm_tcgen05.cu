@@ -181,15 +181,19 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
-  // the raw-weight producer's position in its span; thread 0 carries it across the dependency wait
+  __syncwarp();
+  // the raw-weight producer's position in its span; warp 0 carries it across the dependency wait
   int p_rs = 0, p_u = u0, p_tile = u0 / n_raw, p_rb = u0 % n_raw;
   uint32_t p_phase = 0;
   auto issue_raw = [&]() {  // requests unit p_u's codes and scales into ring slot p_rs and advances
-    mbar_expect_tx(raw_full(p_rs), (uint32_t)kRawStage);
     const uint32_t dst = raw_base + p_rs * kRawStage;
     const int kk = p_rb * kRawK;
-    tma_load_2d(dst, &map_codes, raw_full(p_rs), kk / 2, p_tile * kWRows);
-    tma_load_2d(dst + kRawCodes, &map_scales, raw_full(p_rs), kk / 32, p_tile * kWRows);
+    if (elect_one()) {
+      mbar_expect_tx(raw_full(p_rs), (uint32_t)kRawStage);
+      tma_load_2d(dst, &map_codes, raw_full(p_rs), kk / 2, p_tile * kWRows);
+      tma_load_2d(dst + kRawCodes, &map_scales, raw_full(p_rs), kk / 32, p_tile * kWRows);
+    }
+    __syncwarp();
     if (++p_rs == kRawStages) { p_rs = 0; p_phase ^= 1u; }
     if (++p_rb == n_raw) { p_rb = 0; ++p_tile; }
     ++p_u;
@@ -200,7 +204,7 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   // stages of half a unit) an early-filled ring made about one launch in a few hundred run into an
   // expired wait in a stress test (vocabulary-sized matrix, back-to-back launches); the cause is not
   // understood, and without the early fill 12000 such launches passed.
-  if (w_static && NT <= 64 && threadIdx.x == 0)
+  if (w_static && NT <= 64 && warp == 0)
     while (p_u < u1 && p_u - u0 < kRawStages) issue_raw();
   lg::pdl_wait();  // everything before this touched shared memory or read the static weights only
   if (warp == 2) {
@@ -214,17 +218,15 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 
   if (warp == 0) {
     // ---------------- raw int4 producer ----------------
-    if (lane == 0) {
-      while (p_u < u1) {
-        if (!mbar_wait_sleep(raw_empty(p_rs), p_phase ^ 1u, abort_flag, 100)) break;
-        QTRACE(p_u - u0, 0);
-        issue_raw();
-      }
+    while (p_u < u1) {
+      if (!mbar_wait_sleep_warp(raw_empty(p_rs), p_phase ^ 1u, abort_flag, 100)) break;
+      if (lane == 0) QTRACE(p_u - u0, 0);
+      issue_raw();
     }
   } else if (warp == 1) {
     // ---------------- activation producer: its own ring of 32 KB stages (one barrier per stage), so
     // that the L2 latency of the activations stays off the critical path ----------------
-    if (lane == 0) {
+    {
       int as = 0;
       uint32_t aphase = 0;
       bool ok = true;
@@ -234,12 +236,15 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
         if (++rb == n_raw) rb = 0;
 #pragma unroll
         for (int h = 0; h < kGroups / C::kABlocksPerStage; ++h) {
-          if (!mbar_wait_sleep(a_empty(as), aphase ^ 1u, abort_flag, 100)) { ok = false; break; }
-          if (h == 0) QTRACE(u - u0, 10);
-          mbar_expect_tx(a_full(as), (uint32_t)C::kAStage);
+          if (!mbar_wait_sleep_warp(a_empty(as), aphase ^ 1u, abort_flag, 100)) { ok = false; break; }
+          if (h == 0 && lane == 0) QTRACE(u - u0, 10);
+          if (elect_one()) {
+            mbar_expect_tx(a_full(as), (uint32_t)C::kAStage);
 #pragma unroll
-          for (int b = 0; b < C::kABlocksPerStage; ++b)
-            tma_load_2d(a_base + as * C::kAStage + b * C::kABlock, &map_a, a_full(as), kk + (h * C::kABlocksPerStage + b) * kKB, 0);
+            for (int b = 0; b < C::kABlocksPerStage; ++b)
+              tma_load_2d(a_base + as * C::kAStage + b * C::kABlock, &map_a, a_full(as), kk + (h * C::kABlocksPerStage + b) * kKB, 0);
+          }
+          __syncwarp();
           if (++as == C::kAStages) { as = 0; aphase ^= 1u; }
         }
       }
@@ -249,7 +254,7 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     // own accumulators (the epilogue adds them up). Issuing an MMA or a commit costs a thread on the
     // order of a hundred cycles whatever the tile size, so the k blocks of a unit are issued in
     // parallel by threads on different schedulers; descriptors are built from constants and one add.
-    if (lane == 0) {
+    {
       const int is = warp < 4 ? warp - 2 : warp - 26;
       constexpr uint32_t idesc = make_idesc<NT>();
       constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024 B, version 1, 128-byte swizzle
@@ -269,33 +274,40 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
         const uint32_t tphase = (uint32_t)(seg / C::kAccBufs) & 1u;
         const uint32_t wphase = ((uint32_t)n_unit >> 1) & 1u;
         if (seg_start) {
-          if (!mbar_wait(tempty(buf), tphase ^ 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(tempty(buf), tphase ^ 1u, abort_flag)) { ok = false; break; }
           tc_fence_after();
         }
-        if (is == 0) QTRACE(u - u0, 11);
+        if (is == 0 && lane == 0) QTRACE(u - u0, 11);
         const uint32_t d_tmem = tmem_base + (uint32_t)(C::kAccCol + (is * C::kAccBufs + buf) * NT);
         const int as = ai % C::kAStages;
-        if (!mbar_wait(a_full(as), (uint32_t)(ai / C::kAStages) & 1u, abort_flag)) { ok = false; break; }
-        if (is == 0) QTRACE(u - u0, 6);
+        if (!mbar_wait_warp(a_full(as), (uint32_t)(ai / C::kAStages) & 1u, abort_flag)) { ok = false; break; }
+        if (is == 0 && lane == 0) QTRACE(u - u0, 6);
 #pragma unroll
         for (int j = 0; j < kMine; ++j) {
           const int g = is * kMine + j;
-          if (!mbar_wait(wd_full(wb, g), wphase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(wd_full(wb, g), wphase, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          if (is == 0 && j == 0) QTRACE(u - u0, 7);
+          if (is == 0 && j == 0 && lane == 0) QTRACE(u - u0, 7);
           const uint32_t w_tmem = tmem_base + (uint32_t)(wb * C::kWBufCols + g * kWdCols);  // 8 columns per 16 values of k
           const uint32_t a_lo = a_lo0 + (uint32_t)(as * (C::kAStage >> 4) + (g % per) * (C::kABlock >> 4));
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kKB / 16; ++k)
-            tc_mma_bf16_ts(d_tmem, w_tmem + 8u * k, ((uint64_t)desc_hi << 32) | (a_lo + 2u * k), idesc, (!seg_start || j || k) ? 1u : 0u);
+            for (int k = 0; k < kKB / 16; ++k)
+              tc_mma_bf16_ts(d_tmem, w_tmem + 8u * k, ((uint64_t)desc_hi << 32) | (a_lo + 2u * k), idesc, (!seg_start || j || k) ? 1u : 0u);
+          }
+          __syncwarp();
         }
         if (!ok) break;
-        if (is == 0) QTRACE(u - u0, 8);
-        tc_commit(a_empty(as));
-        tc_commit(wd_empty(wb));
-        if (is == 0) QTRACE(u - u0, 9);
+        if (is == 0 && lane == 0) QTRACE(u - u0, 8);
+        if (elect_one()) {
+          tc_commit(a_empty(as));
+          tc_commit(wd_empty(wb));
+          if (seg_end) tc_commit(tfull(is, buf));
+        }
+        __syncwarp();
+        if (is == 0 && lane == 0) QTRACE(u - u0, 9);
         ai += per == kGroups ? 1 : kIssuers;
-        if (seg_end) { tc_commit(tfull(is, buf)); ++seg; }
+        if (seg_end) ++seg;
       }
     }
   } else if (warp >= 4 && warp < 4 + kDqWarps) {
