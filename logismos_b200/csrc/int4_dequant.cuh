@@ -8,13 +8,18 @@
 
 namespace lg {
 
+// The two masks of an unpacking, kept in registers by the warp (see and_xor).
+struct NibMasks {
+  uint32_t keep = opaque(0x000f000fu), flip = opaque(0x43084308u);
+};
+
 // two nibbles of byte p of a code word (k even in the low nibble) -> bf16x2 {136 + q_even, 136 + q_odd}:
 // the permute puts byte p of w under bits 0-7 and byte p of w >> 4 under bits 16-23; one logic op
 // keeps the two low nibbles, flips their sign bit and ors in the exponent 0x4300
-LG_DEVINL uint32_t nib_pair_136(uint32_t w, uint32_t w_shr4, uint32_t sel) {
+LG_DEVINL uint32_t nib_pair_136(uint32_t w, uint32_t w_shr4, uint32_t sel, const NibMasks& nm) {
   uint32_t t;
   asm("prmt.b32 %0, %1, %2, %3;\n" : "=r"(t) : "r"(w), "r"(w_shr4), "r"(sel));
-  return (t & 0x000f000fu) ^ 0x43084308u;
+  return and_xor(t, nm.keep, nm.flip);
 }
 
 LG_DEVINL uint32_t bf16x2_sub_mul(uint32_t v, uint32_t c136, uint32_t s2) {
@@ -26,14 +31,14 @@ LG_DEVINL uint32_t bf16x2_sub_mul(uint32_t v, uint32_t c136, uint32_t s2) {
 }
 
 // 8 codes of one 32-bit word -> 8 bf16 (one 16-byte chunk of the operand tile), scaled
-LG_DEVINL uint4 dequant_word(uint32_t w, uint32_t s2) {
+LG_DEVINL uint4 dequant_word(uint32_t w, uint32_t s2, const NibMasks& nm) {
   const uint32_t c136 = 0x43084308u;
   const uint32_t lo = w, hi = w >> 4;
   uint4 o;
-  o.x = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0400u), c136, s2);  // bytes {lo.b0, x, hi.b0, x}
-  o.y = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0501u), c136, s2);
-  o.z = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0602u), c136, s2);
-  o.w = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0703u), c136, s2);
+  o.x = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0400u, nm), c136, s2);  // bytes {lo.b0, x, hi.b0, x}
+  o.y = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0501u, nm), c136, s2);
+  o.z = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0602u, nm), c136, s2);
+  o.w = bf16x2_sub_mul(nib_pair_136(lo, hi, 0x0703u, nm), c136, s2);
   return o;
 }
 

@@ -312,9 +312,18 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     }
   } else if (warp >= 4 && warp < 4 + kDqWarps) {
     // ---------------- dequantise: warp group g owns k block g of every unit ----------------
+    // These warps are what bounds the kernel: a unit takes as long as they need for its instructions and waits, whatever the token count up to 64. They test a
+    // barrier some times before they sleep on it (151936 x 1536 at 32 rows: 53.4 -> 49.2 us) and unpack with one logic operation in place of two (-> 43.9).
+    auto wait_dq = [&](uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+      for (int i = 0; i < 16; ++i)
+        if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+      return mbar_wait_sleep_warp(bar, parity, abort_flag);
+    };
     const int wd = warp - 4;
     const int g = wd >> 2;
     const int row = (wd & 3) * 32 + lane;   // weight row of the tile
+    const NibMasks nm;
     int rs = 0, n_unit = 0;
     uint32_t rphase = 0;
     bool ok = true;
@@ -323,7 +332,7 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
       const int wb = n_unit & 1;
       const uint32_t wphase = ((uint32_t)n_unit >> 1) & 1u;
       if (wd == 0 && lane == 0) QTRACE(u - u0, 1);
-      if (!mbar_wait_sleep_warp(raw_full(rs), rphase, abort_flag)) { ok = false; break; }
+      if (!wait_dq(raw_full(rs), rphase)) { ok = false; break; }
       if (wd == 0 && lane == 0) QTRACE(u - u0, 2);
       const uint8_t* raw = smem_gen + rs * kRawStage;
       // this row's 64 codes of k block g (two 16-byte chunks, swizzled by the TMA) and their two scales
@@ -335,10 +344,10 @@ qlinear_int4_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __g
       if (++rs == kRawStages) { rs = 0; rphase ^= 1u; }
       const uint32_t s0 = scale_bf16x2(sc, 0), s1 = scale_bf16x2(sc, 1);
       uint4 o[8];
-      o[0] = dequant_word(c0.x, s0); o[1] = dequant_word(c0.y, s0); o[2] = dequant_word(c0.z, s0); o[3] = dequant_word(c0.w, s0);
-      o[4] = dequant_word(c1.x, s1); o[5] = dequant_word(c1.y, s1); o[6] = dequant_word(c1.z, s1); o[7] = dequant_word(c1.w, s1);
+      o[0] = dequant_word(c0.x, s0, nm); o[1] = dequant_word(c0.y, s0, nm); o[2] = dequant_word(c0.z, s0, nm); o[3] = dequant_word(c0.w, s0, nm);
+      o[4] = dequant_word(c1.x, s1, nm); o[5] = dequant_word(c1.y, s1, nm); o[6] = dequant_word(c1.z, s1, nm); o[7] = dequant_word(c1.w, s1, nm);
       if (wd == 0 && lane == 0) QTRACE(u - u0, 3);
-      if (!mbar_wait_sleep_warp(wd_empty(wb), wphase ^ 1u, abort_flag)) { ok = false; break; }
+      if (!wait_dq(wd_empty(wb), wphase ^ 1u)) { ok = false; break; }
       tc_fence_after();
       if (wd == 0 && lane == 0) QTRACE(u - u0, 4);
       tc_st32(wt0 + (uint32_t)(wb * C::kWBufCols), o);  // lane = weight row, 32 columns = its 64 bf16 in k order
