@@ -52,7 +52,23 @@ struct Cfg {
   static constexpr size_t kSmem = (size_t)kStages * kStage + kEpiBytes + 1024 /*align*/ + 256 /*barriers*/;
 };
 
-LG_DEVINL float silu_f(float x) { return x / (1.0f + __expf(-x)); }
+// x / (1 + exp(-x)), a rounded division here and in int4_rows. LATENCY: the quotient by Markstein's correction (q + r * (x - q * d), IBM J. Res. Dev. 34,
+// 1990) in place of the operator, whose branches keep the quotients of a row from overlapping; the same bits but for 2 of 1.8e9 floats, which differ in the last. Where d or
+// x is infinite the remainder is NaN and the first quotient is the answer. For tiles of 128 columns, which calls of few rows take and whose last epilogue nothing hides: it took 4100 cycles
+// with the operator (17920 x 1536 at 17 rows 17.8 -> 15.7 us, 12288 x 2048 at 64 17.2 -> 15.7, with the early requests below). Larger tiles hide it behind the next tile's MMAs, and there the
+// additional operations cost more than the branches: 861 against 885 us for 17920 x 1536 at 20 thousand rows, by pairs.
+template <bool LATENCY>
+LG_DEVINL float silu_f(float x) {
+  float d = 1.0f + __expf(-x);
+  if (!LATENCY) return x / d;
+  const float scale = d > 0x1p100f ? 0x1p-64f : 1.0f;  // the reciprocal of a d above 2^126 would be flushed to zero
+  x *= scale;
+  d *= scale;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(d));
+  const float q = x * r, rem = fmaf(-q, d, x), fixed = fmaf(rem, r, q);
+  return rem == rem ? fixed : q;
+}
 
 // eight bias values (the same for every lane); vec: the pointer is 16-byte aligned
 LG_DEVINL void load_bias8(const float* __restrict__ bias, bool vec, float (&b)[8]) {
@@ -150,6 +166,10 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_gen + 8 * (2 * C::kStages + 4) + 8);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 1 && elect_one()) {  // the descriptors are on their way while the preceding kernel drains
+    prefetch_map(&map_a);
+    prefetch_map(&map_out);
+  }
   if (EXPERTS) lg::pdl_wait();  // the tile list is the work of a kernel of this step
   const int rank = PAIR ? (int)cluster_rank() : 0;  // 0 issues the MMAs of a pair
   const int first_tile = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, tile_step = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
@@ -169,10 +189,7 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
   __syncwarp();
-  // w_static: nothing still in flight writes the weights, so the weight halves of the first stages of
-  // this CTA's first tile are requested before the dependency wait (they land while the preceding
-  // kernel drains); each stage's barrier already expects the bytes of both halves
-  int pre_w = 0;
+  // w_static: nothing still in flight writes the weights
   if (PAIR) cluster_sync();  // the barriers of both CTAs are there
   // a stage of a pair is complete when the bytes of both CTAs have arrived at the first one's barrier
   auto expect_stage = [&](int s) { if (rank == 0) mbar_expect_tx(full_bar(s), (uint32_t)C::kStage * (PAIR ? 2u : 1u)); };
@@ -180,20 +197,34 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     if (PAIR) tma_load_2d_pair(dst, map, peer_smem(full_bar(s), 0), x, y);
     else tma_load_2d(dst, map, full_bar(s), x, y);
   };
-  if (w_static && warp == 0 && first_tile < total_tiles) {
+  // The first stages of this CTA's first tile: their weights before the dependency wait, their activations (and weights that are not static) right after it and
+  // before the wait for tensor memory.
+  int pre = 0;  // stages that need nothing more from the producer's loop
+  if (!EXPERTS && warp == 0 && first_tile < total_tiles) {
     const int ot = first_tile % out_tiles, sp = first_tile / out_tiles;
     int m_blk, n_blk;
     tile_at(ot, m_tiles, n_tiles, group, m_blk, n_blk);
-    const int kb0 = sp * kb_per, kb1 = min(all_kb, kb0 + kb_per);
-    for (int kb = kb0; kb < kb1 && pre_w < C::kStages; ++kb, ++pre_w) {
+    const int kb0 = sp * kb_per, n_pre = min(min(all_kb, kb0 + kb_per) - kb0, C::kStages);
+    const int w_row = n_blk * BN + rank * C::kRowsB, a_row = m_blk * kTileM + rank * BM + (EPI == kEpiGroups ? group_of(groups, n_blk * BN) * M : 0);
+    auto weights = [&](int s) {
+      expect_stage(s);
+      load(smem_base + s * C::kStage + C::kStageA, &map_w, s, (kb0 + s) * BK, w_row);
+    };
+    for (int s = 0; w_static && s < n_pre; ++s) {
+      if (elect_one()) weights(s);
+      __syncwarp();
+    }
+    lg::pdl_wait();
+    for (; pre < n_pre; ++pre) {
       if (elect_one()) {
-        expect_stage(pre_w);
-        load(smem_base + pre_w * C::kStage + C::kStageA, &map_w, pre_w, kb * BK, n_blk * BN + rank * C::kRowsB);
+        if (!w_static) weights(pre);
+        load(smem_base + pre * C::kStage, &map_a, pre, (kb0 + pre) * BK, a_row);
       }
       __syncwarp();
     }
+  } else if (!EXPERTS) {
+    lg::pdl_wait();  // everything before this touched shared memory or read the static weights only
   }
-  if (!EXPERTS) lg::pdl_wait();  // everything before this touched shared memory or read the static weights only
   if (warp == 1) {
     if (PAIR) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32((const void*)tmem_slot)), "r"((uint32_t)C::kTmemCols) : "memory");
@@ -231,16 +262,18 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
           if (direct) a_map = &map_out;
         }
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
-          const bool have_w = pre_w > 0;  // requested before the dependency wait (first stages of the first tile)
-          const uint32_t sa = smem_base + stage * C::kStage;
-          if (elect_one()) {
-            if (!have_w) expect_stage(stage);
-            load(sa, a_map, stage, kb * BK, a_row);
-            if (!have_w) load(sa + C::kStageA, &map_w, stage, kb * BK, w_row);
+          if (pre > 0) {
+            --pre;
+          } else {
+            if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
+            const uint32_t sa = smem_base + stage * C::kStage;
+            if (elect_one()) {
+              expect_stage(stage);
+              load(sa, a_map, stage, kb * BK, a_row);
+              load(sa + C::kStageA, &map_w, stage, kb * BK, w_row);
+            }
+            __syncwarp();
           }
-          if (have_w) --pre_w;
-          __syncwarp();
           if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -470,7 +503,7 @@ linear_t_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 const float g0 = __uint_as_float(g[e]) + bg[2 * i], g1 = __uint_as_float(g[e + 1]) + bg[2 * i + 1];
                 const float u0 = __uint_as_float(u[e]) + bu[2 * i], u1 = __uint_as_float(u[e + 1]) + bu[2 * i + 1];
                 if (EPI == LG_EPI_GLU_CLAMP) w[i] = pack_bf16x2(lg::glu_clamp(g0, u0, ep.p0, ep.p1, ep.p2), lg::glu_clamp(g1, u1, ep.p0, ep.p1, ep.p2));
-                else w[i] = pack_bf16x2(silu_f(g0) * u0, silu_f(g1) * u1);  // a rounded division, here and in int4_rows
+                else w[i] = pack_bf16x2(silu_f<BN == 128>(g0) * u0, silu_f<BN == 128>(g1) * u1);
               }
               *reinterpret_cast<uint4*>(dst + j * 8) = make_uint4(w[0], w[1], w[2], w[3]);
             }

@@ -103,6 +103,7 @@ LG_DEVINL bool mbar_wait_sleep_warp(uint32_t bar, uint32_t parity, volatile int*
   return __all_sync(0xffffffffu, mbar_wait_sleep(bar, parity, abort_flag, ns)) != 0;
 }
 
+LG_DEVINL void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory"); }
 LG_DEVINL void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
