@@ -192,6 +192,9 @@ LG_DEVINL uint32_t opaque(uint32_t v) {
   return r;
 }
 
+// a hint only: what is read later is what memory holds then
+LG_DEVINL void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
 // 16-byte async copy global -> shared, bypassing L1 (data is streamed once).
 LG_DEVINL void cp_async16(uint32_t smem_addr, const void* gptr) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr), "l"(gptr));

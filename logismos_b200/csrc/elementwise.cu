@@ -35,24 +35,29 @@ __global__ void embed_lookup_kernel(const __nv_bfloat16* __restrict__ table,
 
 // cpu_f32::rms_norm (mod.rs:137-159). One CTA per row, the row held in registers between the
 // two passes (n <= 8 * 4 * blockDim).
+// Rows of a decode step: what counts is the chain of round trips. The gains, which a pass over the weights has pushed out to HBM since the last step, are
+// fetched into L2 ahead of the dependency wait and requested together with the row, not behind its sum: 64 rows of 2048 in a decode step 4.4 -> 3.3 us.
 template <bool OUT_F32>
 __global__ void rms_norm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                     void* __restrict__ y, int n, float eps) {
-  lg::pdl_prologue();
+  lg::pdl_trigger();
+  for (int j = threadIdx.x * 4; j < n; j += blockDim.x * 4) prefetch_l2(w + j);
+  lg::pdl_wait();
   __shared__ float red[32];
   const float* row = x + (size_t)blockIdx.x * n;
-  float4 v[8];
+  float4 v[8], g8[8];
   float ss = 0.0f;
   int cnt = 0;
   for (int j = threadIdx.x * 4; j < n && cnt < 8; j += blockDim.x * 4, ++cnt) {
     v[cnt] = *reinterpret_cast<const float4*>(row + j);
+    g8[cnt] = __ldg(reinterpret_cast<const float4*>(w + j));
     ss += v[cnt].x * v[cnt].x + v[cnt].y * v[cnt].y + v[cnt].z * v[cnt].z + v[cnt].w * v[cnt].w;
   }
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)n + eps);
   cnt = 0;
   for (int j = threadIdx.x * 4; j < n && cnt < 8; j += blockDim.x * 4, ++cnt) {
-    const float4 g = __ldg(reinterpret_cast<const float4*>(w + j));
+    const float4 g = g8[cnt];
     const float o0 = v[cnt].x * inv * g.x, o1 = v[cnt].y * inv * g.y;
     const float o2 = v[cnt].z * inv * g.z, o3 = v[cnt].w * inv * g.w;
     if (OUT_F32) {
@@ -70,15 +75,18 @@ __global__ void rms_norm_f32_kernel(const float* __restrict__ x, const float* __
 template <bool OUT_F32>
 __global__ void __launch_bounds__(512)
 rms_norm_parts_kernel(float* __restrict__ x, const float* __restrict__ parts, int slices, size_t part, const float* __restrict__ w, void* __restrict__ y, int n, float eps) {
-  lg::pdl_prologue();
+  lg::pdl_trigger();
+  for (int j = threadIdx.x * 4; j < n; j += blockDim.x * 4) prefetch_l2(w + j);
+  lg::pdl_wait();
   __shared__ float red[32];
   float* row = x + (size_t)blockIdx.x * n;
   const float* own = parts + (size_t)blockIdx.x * n;
-  float4 v[4];
+  float4 v[4], g4[4];
   float ss = 0.0f;
   int cnt = 0;
   for (int j = threadIdx.x * 4; j < n && cnt < 4; j += blockDim.x * 4, ++cnt) {
     float4 a = *reinterpret_cast<const float4*>(row + j);
+    g4[cnt] = __ldg(reinterpret_cast<const float4*>(w + j));
 #pragma unroll 6
     for (int s = 0; s < slices; ++s) {
       const float4 b = *reinterpret_cast<const float4*>(own + (size_t)s * part + j);
@@ -92,7 +100,7 @@ rms_norm_parts_kernel(float* __restrict__ x, const float* __restrict__ parts, in
   const float inv = 1.0f / sqrtf(ss / (float)n + eps);
   cnt = 0;
   for (int j = threadIdx.x * 4; j < n && cnt < 4; j += blockDim.x * 4, ++cnt) {
-    const float4 g = __ldg(reinterpret_cast<const float4*>(w + j));
+    const float4 g = g4[cnt];
     const float o0 = v[cnt].x * inv * g.x, o1 = v[cnt].y * inv * g.y, o2 = v[cnt].z * inv * g.z, o3 = v[cnt].w * inv * g.w;
     if (OUT_F32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + (size_t)blockIdx.x * n + j) = make_float4(o0, o1, o2, o3);
     else *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(y) + (size_t)blockIdx.x * n + j) = make_uint2(pack_bf16x2(o0, o1), pack_bf16x2(o2, o3));
