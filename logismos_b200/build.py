@@ -29,7 +29,7 @@ CU_SOURCES = ["cudacore.cu", "legacy_fp16.cu", "elementwise.cu", "gemv_int4.cu",
               "linear_small.cu", "depth_conv.cu", "latent_attention.cu", "latent_model.cu",
               "post_norm.cu", "tanh_norm.cu", "time_mix.cu", "ssd.cu", "bias_attention.cu", "rotary.cu", "moe.cu", "mixer_parallel.cu",
               "gated_residual.cu", "mixer_gated.cu", "mixer_paired.cu", "mixer_model.cu"]
-CPP_SOURCES = ["sched.cpp", "loader.cpp", "checkpoints.cpp"]
+CPP_SOURCES = ["decode_plan.cpp", "sched.cpp", "loader.cpp", "checkpoints.cpp"]
 
 # what one model family needs: the sources of a library that serves it alone
 GROUPS = {

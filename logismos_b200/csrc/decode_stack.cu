@@ -24,8 +24,6 @@
 // fp32 on the finished group; the sums of the warps are added in shared memory in order. Nothing is added without an order, so results repeat.
 #include "decode_stack.h"
 
-#include <algorithm>
-
 #include "common.cuh"
 #include "decode_tiles.cuh"
 #include "int4_rows.h"
@@ -35,16 +33,11 @@ namespace lg {
 namespace {
 
 using namespace tc;
+using namespace stack;
 
-constexpr int kDim = 128, kMaxWarps = 12, kBringers = 1, kMaxChunks = 32, kStage = 2 * kBlock * kDim * 2;
+constexpr int kBringers = 1;
+static_assert(kTokens == kBlock, "cache blocks");
 constexpr uint32_t kPolls = 1u << 20;  // of a word: about a second
-
-enum { kQkv, kOut, kGateUp, kDown, kMats };
-
-__host__ __device__ constexpr int round_up(int v, int to) { return (v + to - 1) / to * to; }
-// a row of codes in shared memory: rows lie 16 bytes apart modulo the banks, so that eight rows' words of a group meet no conflict
-__host__ __device__ constexpr int code_stride(int k) { return round_up(k / 2, 128) + 16; }
-__host__ __device__ constexpr int row_bytes(int k) { return code_stride(k) + k / 16; }
 
 struct Kernel {
   StackArgs a;
@@ -578,7 +571,11 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
   }
   if (tid < kLayerWords) reinterpret_cast<uint64_t*>(s_layer)[tid] = layer_word(0);
   const uint32_t parts = p.at_part;
-  for (uint32_t i = 4u * tid; i < (uint32_t)(round_up(warps, 4) - warps) * p.part_step; i += 4u * blockDim.x) sts(parts + warps * p.part_step + i, 0.0f);
+  // the parts of warps that are not there are zero whenever sums are taken: what else goes to their place is cleared again
+  auto clear_tail = [&](int n) {
+    for (uint32_t i = 4u * tid; i < (uint32_t)(round_up(warps, 4) - warps) * p.part_step; i += 4u * n) sts(parts + warps * p.part_step + i, 0.0f);
+  };
+  clear_tail(blockDim.x);
   __syncthreads();
 
   // rows of this CTA and what they are, the same in every layer
@@ -722,6 +719,7 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
     if (meet_any(threads, s_abort)) break;
 #pragma unroll 1
     for (int t = p.ctas - 1 - cta; t < merges; t += p.ctas) merge(kern, s_mail, number, &s_abort, t / n_heads, t % n_heads, parts);
+    if (p.ctas - 1 - cta < merges) clear_tail(threads);  // where a warp's part is smaller than its room, the rooms reach there
 
     gain = load4_now(L.norm2 + 4 * tid);
 
@@ -829,78 +827,6 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
 }
 
 }  // namespace
-
-bool stack_plan(const StackDims& d, StackPlan* plan) {
-  const int H = d.hidden, I = d.inter, R = d.rows;
-  if (R < 1 || R > kFewRows || H % 256 || I % 256 || H / kDim > kMaxWarps || d.n_heads * kDim != H || d.n_kv < 1 || d.n_heads % d.n_kv || d.n_heads / d.n_kv > 8) return false;
-  StackPlan p{};
-  p.ctas = sm_count();
-  p.warps = H / kDim;
-  auto share = [&](int n) { return (n + p.ctas - 1) / p.ctas; };
-  p.qkv_tiles = share((d.n_heads + 2 * d.n_kv) * (kDim / 16));
-  p.gu_tiles = share(I / 8);
-  p.out_rows = share(H);
-  p.max_chunks = std::max(1, std::min(kMaxChunks, p.ctas / (R * d.n_kv)));
-  const int rp = R == 1 ? 1 : R == 2 ? 2 : 4, out_tiles = (p.out_rows + 15) / 16, rep = d.n_heads / d.n_kv;
-  auto align = [](size_t v) { return (v + 127) & ~(size_t)127; };
-  p.at[kGateUp] = 0;
-  size_t at = align(std::max((size_t)16 * p.gu_tiles * row_bytes(H), (size_t)R * (I + 32) * 2 + (size_t)(I / 32) * 16));
-  p.at[kDown] = (uint32_t)at;
-  // cached blocks and the sums of their warps lie where the down projection's rows come next
-  const size_t down = (size_t)p.out_rows * row_bytes(I), per_warp = std::max((size_t)kStage, (size_t)rep * (kDim + 6) * 4);
-  p.att_warps = std::min(p.warps, std::max(2, (int)(down / per_warp)));
-  at += align(std::max(down, p.att_warps * per_warp));
-  p.at[kQkv] = (uint32_t)at;
-  at += align((size_t)16 * p.qkv_tiles * row_bytes(H));
-  p.at[kOut] = (uint32_t)at;
-  at += align((size_t)p.out_rows * row_bytes(H));
-  p.at_x = (uint32_t)at;
-  at += align((size_t)R * (H + 32) * 2);
-  p.at_turn = (uint32_t)at;
-  at += align((size_t)8 * p.qkv_tiles * R * 16);
-  p.at_sums = (uint32_t)at;
-  at += align((size_t)(H / 32) * 16);
-  p.at_part = (uint32_t)at;  // and the chunks that a CTA puts together
-  p.part_step = (uint32_t)(16 * std::max({p.gu_tiles, p.qkv_tiles, out_tiles}) * rp * 4);
-  at += align(std::max((size_t)round_up(p.warps, 4) * p.part_step, (size_t)p.warps * kDim * 4));
-  p.bytes = (uint32_t)at;
-  p.at_scales[kQkv] = p.at[kQkv] + 16 * p.qkv_tiles * code_stride(H);
-  p.at_scales[kOut] = p.at[kOut] + p.out_rows * code_stride(H);
-  p.at_scales[kGateUp] = 16 * p.gu_tiles * code_stride(H);
-  p.at_scales[kDown] = p.at[kDown] + p.out_rows * code_stride(I);
-  // tiles that end in rows which are not there read up to 15 rows on
-  for (int m : {kOut, kDown}) {
-    const int k = m == kOut ? H : I;
-    p.bytes = std::max({p.bytes, p.at[m] + 16 * out_tiles * code_stride(k), p.at_scales[m] + 16 * out_tiles * (k / 16)});
-  }
-  const int threads = 32 * p.warps;  // one for each pair of q, k, v and for each value of the projections
-  if (p.bytes > 226 * 1024 || 8 * p.qkv_tiles * R > threads || p.out_rows * R > threads || sizeof(StackLayer) / 8 > (size_t)threads) return false;
-  *plan = p;
-  return true;
-}
-
-int stack_chunk(const StackPlan& plan, const int32_t* ctx, int rows) {
-  int longest = 1;
-  for (int r = 0; r < rows; ++r) longest = std::max(longest, ctx[r]);
-  const int least = (longest + plan.max_chunks - 1) / plan.max_chunks;
-  return std::max(round_up(least, kBlock), kBlock * plan.att_warps);
-}
-
-bool stack_blocks_apart(const int32_t* tables, int max_blocks, const int32_t* ctx, int rows) {
-  for (int r = 0; r < rows; ++r) {
-    const int last = (ctx[r] - 1) / kBlock;
-    if (ctx[r] < 1 || last >= max_blocks) return false;
-    for (int s = 0; s < rows; ++s)
-      for (int b = 0; b < max_blocks && b * kBlock < ctx[s]; ++b)
-        if (tables[(size_t)s * max_blocks + b] == tables[(size_t)r * max_blocks + last] && !(s == r && b == last)) return false;
-  }
-  return true;
-}
-
-size_t stack_words(const StackDims& d) {
-  const size_t R = (size_t)d.rows, heads = (size_t)d.n_heads;
-  return R * ((heads + 2 * d.n_kv) * (kDim / 2) + heads * kMaxChunks * (kDim + 2) + heads * (kDim / 2) + 2 * (size_t)d.hidden + d.inter / 2);
-}
 
 uint32_t launch_decode_stack(const StackArgs& a, const StackPlan& plan, cudaStream_t stream) {
   if (a.n_layers <= 0) return 0;

@@ -7,6 +7,16 @@
 
 namespace lg {
 
+namespace stack {
+constexpr int kDim = 128, kMaxWarps = 12, kMaxChunks = 32, kTokens = 16 /* of a cache block */, kStage = 2 * kTokens * kDim * 2;
+enum { kQkv, kOut, kGateUp, kDown, kMats };
+
+__host__ __device__ constexpr int round_up(int v, int to) { return (v + to - 1) / to * to; }
+// a row of codes in shared memory: rows lie 16 bytes apart modulo the banks, so that eight rows' words of a group meet no conflict
+__host__ __device__ constexpr int code_stride(int k) { return round_up(k / 2, 128) + 16; }
+__host__ __device__ constexpr int row_bytes(int k) { return code_stride(k) + k / 16; }
+}  // namespace stack
+
 struct StackMat {
   const uint8_t* codes;  // [n][k / 2]
   const __half* scales;  // [n][k / 32]
@@ -29,7 +39,7 @@ struct StackPlan {
   // offsets of the parts of shared memory: rows of q, k, v | output | gate, up | down and their scales, activations, angles of q, k, v, sums of activations, the warps' sums (part_step bytes each)
   uint32_t at[4], at_scales[4], at_x, at_turn, at_sums, at_part, part_step, bytes;
 };
-bool stack_plan(const StackDims& d, StackPlan* plan);
+bool stack_plan(const StackDims& d, int ctas, StackPlan* plan);
 // tokens per chunk of the longest of `rows` contexts
 int stack_chunk(const StackPlan& plan, const int32_t* ctx, int rows);
 // No row's new token goes to a block that another row, or another place of its own table, holds: blocks without a new token may be read before it is stored.

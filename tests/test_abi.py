@@ -203,3 +203,15 @@ def test_rows_to_the_host_call_cuda_from_one_thread(tmp_path):
                            os.path.join(here, "host_rows_check.cpp"), "-o", exe])
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_layouts_of_the_one_launch_decode_step(tmp_path):
+    """Every layout that stack_plan accepts: parts of shared memory that are live together lie apart, within the launch's bytes and aligned; every weight row has a CTA."""
+    import os
+    import subprocess
+    here = os.path.dirname(os.path.abspath(__file__))
+    root, exe = os.path.dirname(here), str(tmp_path / "decode_plan")
+    csrc, cuda = os.path.join(root, "logismos_b200", "csrc"), os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-I" + csrc, "-I" + os.path.join(cuda, "include"), os.path.join(here, "decode_plan_check.cpp"), os.path.join(csrc, "decode_plan.cpp"), "-o", exe])
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -214,6 +214,36 @@ def test_one_launch_and_one_per_projection_on_long_contexts():
     model.close()
 
 
+@pytest.mark.parametrize("heads,kv,inter", [(10, 2, 3840), (10, 5, 512), (10, 10, 1024), (6, 2, 1024), (2, 1, 256)])
+@pytest.mark.parametrize("n_seqs", [1, 2, 3, 4])
+def test_one_launch_with_warps_that_are_no_multiple_of_four(heads, kv, inter, n_seqs):
+    """Ten, six and two warps, few tiles a CTA and contexts of one to many chunks, so that a CTA puts chunks together and holds weight rows as well: the layers as one launch against
+    the general route of the deterministic switch. Bound: as the tests against the oracle."""
+    from logismos_b200._lib import lib
+    cfg = dict(TINY, hidden=128 * heads, n_heads=heads, n_kv_heads=kv, intermediate=inter, vocab=520, n_layers=3, max_pos=2048)
+    qw, _ = quantize_weights(cfg, make_weights(cfg, 13))
+    model = DecoderModel(cfg, qw, n_pool_blocks=300, max_blocks_per_seq=100, max_step_tokens=1536, max_step_seqs=4)
+    rng, alloc = np.random.default_rng([heads, n_seqs]), BlockAllocator(300, 100, seed=2)
+    lens = [400, 1500, 20, 150]
+    tables = np.stack([alloc.ensure(i, n + 1) for i, n in enumerate(lens)])
+    for i, n in enumerate(lens):
+        model.step(rng.integers(0, 520, n), [0], [n], tables[i:i + 1])
+    for first in range(4):
+        which = [(first + i) % 4 for i in range(n_seqs)]
+        out = []
+        for det in (0, 1):
+            lib.logismos_set_deterministic(det)
+            try:
+                model.step([5 + i for i in which], [lens[i] for i in which], [1] * n_seqs, tables[which])
+                out.append((model.last_hidden().copy(), model.last_logits().copy()))
+                assert (model.launches_last_step() <= 7) == (det == 0)
+            finally:
+                lib.logismos_set_deterministic(0)
+        for i in range(n_seqs):
+            assert max_rel(out[0][0][i], out[1][0][i]) <= TOL and max_rel(out[0][1][i], out[1][1][i]) <= TOL, (first, i)
+    model.close()
+
+
 def test_deterministic_switch_keeps_a_row_independent_of_its_step():
     """With the switch on, a sequence's decode steps have the same bits alone and beside 3, 4 and 29 others: the same projections and the
     same pieces of its context of 1000 tokens."""
