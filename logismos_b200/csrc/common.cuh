@@ -195,13 +195,14 @@ LG_DEVINL uint32_t opaque(uint32_t v) {
 // a hint only: what is read later is what memory holds then
 LG_DEVINL void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 
-// 16-byte async copy global -> shared, bypassing L1 (data is streamed once).
+// 16-byte async copy global -> shared, bypassing L1 (data is streamed once). The clobbers keep plain accesses of shared memory on their side: a copy goes behind
+// the loads of what it overwrites, loads of what it brings go behind the wait. Not every use has a barrier there (a thread may copy for itself alone).
 LG_DEVINL void cp_async16(uint32_t smem_addr, const void* gptr) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr), "l"(gptr));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr), "l"(gptr) : "memory");
 }
-LG_DEVINL void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+LG_DEVINL void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
-LG_DEVINL void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+LG_DEVINL void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // mma.sync m16n8k16, bf16 inputs, fp32 accumulate: D = A(16x16,row) * B(16x8,col) + C
 LG_DEVINL void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2],

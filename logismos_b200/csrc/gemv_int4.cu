@@ -356,7 +356,7 @@ gemv_int4_g32_stream_kernel(const uint8_t* __restrict__ codes, const __half* __r
         cp_async16(p_slot + dst_w + h * 8 * kWPitch, pw[h]);
         pw[h] += 64;
       }
-      if (lane < kRows) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(p_slot + dst_s), "l"(ps));
+      if (lane < kRows) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(p_slot + dst_s), "l"(ps) : "memory");
       ps += 4;
       p_slot += kSlot;
       if (p_slot == ring_end) p_slot = ring;

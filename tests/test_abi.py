@@ -215,3 +215,22 @@ def test_layouts_of_the_one_launch_decode_step(tmp_path):
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-I" + csrc, "-I" + os.path.join(cuda, "include"), os.path.join(here, "decode_plan_check.cpp"), os.path.join(csrc, "decode_plan.cpp"), "-o", exe])
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_asynchronous_copies_and_barriers_are_ordered_for_the_compiler():
+    """Inline instructions that start or await asynchronous copies, or that arrive at a barrier, say that they touch memory: without it the compiler may move plain accesses of the
+    same shared memory across them."""
+    import glob
+    import os
+    import re
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "logismos_b200", "csrc")
+    seen = 0
+    for path in sorted(glob.glob(os.path.join(csrc, "*.cu*")) + glob.glob(os.path.join(csrc, "*.h"))):
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for m in re.finditer(r"\basm\b(?: volatile)?\s*\(", text):
+            body = text[m.start():text.index(");", m.end())]
+            if re.search(r"cp\.(reduce\.)?async|mbarrier\.|tcgen05\.(commit|mma)|barrier\.cluster", body):
+                seen += 1
+                assert '"memory"' in body, (os.path.basename(path), body)
+    assert seen > 20
