@@ -35,29 +35,32 @@ __global__ void embed_lookup_kernel(const __nv_bfloat16* __restrict__ table,
 
 // cpu_f32::rms_norm (mod.rs:137-159). One CTA per row, the row held in registers between the
 // two passes (n <= 8 * 4 * blockDim).
-// Rows of a decode step: what counts is the chain of round trips. The gains, which a pass over the weights has pushed out to HBM since the last step, are
-// fetched into L2 ahead of the dependency wait and requested together with the row, not behind its sum: 64 rows of 2048 in a decode step 4.4 -> 3.3 us.
-template <bool OUT_F32>
+// FEW, the rows of a decode step: what counts is the chain of round trips. The gains, which a pass over the weights has pushed out to HBM since the last step, are
+// fetched into L2 ahead of the dependency wait and requested together with the row, not behind its sum: 64 rows of 2048 in a decode step 4.4 -> 3.3 us. Its
+// registers cost CTAs per SM: up to three rows an SM it is the faster one at every length (0.67 to 1.0 of the other's time), from 500 rows on the slower one (up to
+// 1.4 times as long at 592 rows and more of 1536 to 8192).
+template <bool OUT_F32, bool FEW>
 __global__ void rms_norm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                     void* __restrict__ y, int n, float eps) {
   lg::pdl_trigger();
-  for (int j = threadIdx.x * 4; j < n; j += blockDim.x * 4) prefetch_l2(w + j);
+  if (FEW)
+    for (int j = threadIdx.x * 4; j < n; j += blockDim.x * 4) prefetch_l2(w + j);
   lg::pdl_wait();
   __shared__ float red[32];
   const float* row = x + (size_t)blockIdx.x * n;
-  float4 v[8], g8[8];
+  float4 v[8], g8[FEW ? 8 : 1];
   float ss = 0.0f;
   int cnt = 0;
   for (int j = threadIdx.x * 4; j < n && cnt < 8; j += blockDim.x * 4, ++cnt) {
     v[cnt] = *reinterpret_cast<const float4*>(row + j);
-    g8[cnt] = __ldg(reinterpret_cast<const float4*>(w + j));
+    if (FEW) g8[cnt] = __ldg(reinterpret_cast<const float4*>(w + j));
     ss += v[cnt].x * v[cnt].x + v[cnt].y * v[cnt].y + v[cnt].z * v[cnt].z + v[cnt].w * v[cnt].w;
   }
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)n + eps);
   cnt = 0;
   for (int j = threadIdx.x * 4; j < n && cnt < 8; j += blockDim.x * 4, ++cnt) {
-    const float4 g = g8[cnt];
+    const float4 g = FEW ? g8[FEW ? cnt : 0] : __ldg(reinterpret_cast<const float4*>(w + j));
     const float o0 = v[cnt].x * inv * g.x, o1 = v[cnt].y * inv * g.y;
     const float o2 = v[cnt].z * inv * g.z, o3 = v[cnt].w * inv * g.w;
     if (OUT_F32) {
@@ -410,10 +413,9 @@ uint32_t logismos_launch_rms_norm_f32(const void* x, const void* w, void* y, int
   }
   int bs = 32;
   while (bs * 4 * 2 < n && bs < 256) bs <<= 1;  // aim for ~2 float4 per thread
-  if (out_f32)
-    lg::launch(rms_norm_f32_kernel<true>, dim3(rows), dim3(bs), 0, (cudaStream_t)stream, (const float*)x, (const float*)w, y, n, eps);
-  else
-    lg::launch(rms_norm_f32_kernel<false>, dim3(rows), dim3(bs), 0, (cudaStream_t)stream, (const float*)x, (const float*)w, y, n, eps);
+  const bool few = rows <= 3 * lg::sm_count();
+  auto kern = out_f32 ? few ? rms_norm_f32_kernel<true, true> : rms_norm_f32_kernel<true, false> : few ? rms_norm_f32_kernel<false, true> : rms_norm_f32_kernel<false, false>;
+  lg::launch(kern, dim3(rows), dim3(bs), 0, (cudaStream_t)stream, (const float*)x, (const float*)w, y, n, eps);
   return lg::launch_status();
 }
 

@@ -33,6 +33,17 @@ def test_rms_norm_f32(rows, n):
     assert max_rel(to_np(yb), ref) < 8e-3  # one bf16 rounding
 
 
+@pytest.mark.parametrize("n", [4, 100, 1536, 3072, 8192])
+def test_rms_norm_of_few_and_of_many_rows_gives_the_same_bits(n):
+    """Up to three rows an SM have a kernel of their own (444 of the 445 and more on 148 SMs)."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x, w = torch.randn(1000, n, generator=g, device=DEV), torch.randn(n, generator=g, device=DEV)
+    for out_f32 in (False, True):
+        many = ops.rms_norm_f32(x, w, 1e-6, out_f32=out_f32)
+        for rows in (1, 148, 444, 445):
+            assert torch.equal(ops.rms_norm_f32(x[:rows].contiguous(), w, 1e-6, out_f32=out_f32), many[:rows]), rows
+
+
 @pytest.mark.parametrize("d", [128, 256, 40])  # 40: not a multiple of 16, the narrow-access kernel
 def test_rope_halves_on_packed_qkv_rows(d):
     rng = np.random.default_rng(2)
