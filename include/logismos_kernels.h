@@ -717,7 +717,8 @@ uint32_t logismos_launch_repetition_penalty_f32(void* logits_f32, int32_t rows, 
 uint32_t logismos_launch_multinomial_f32(const void* logits_f32, int32_t rows, int32_t n,
                                          const void* uniforms_f32, void* out_u32, void* stream);
 /* Temperature, top-k, top-p, min-p and the multinomial draw in that order, with the results of the five
- * launchers above (arguments as there; a value that is a no-op there is one here): one launch where 0 < k <= 256. */
+ * launchers above (arguments as there; a value that is a no-op there is one here): one launch where k is small
+ * for n (144 of 2047 values with a top-p, up to 256 of 24576 and more; fewer without). */
 uint32_t logismos_launch_sample_chain_f32(void* logits_f32, int32_t rows, int32_t n, float temperature,
                                           int32_t k, float p, float min_p, const void* uniforms_f32,
                                           void* out_u32, void* stream);

@@ -19,6 +19,8 @@
 // at the cut are kept in index order, as the reference's stable sort does.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "logismos_kernels.h"
 
@@ -38,7 +40,7 @@ static_assert(kSegment == kThreads, "a thread per bin of a segment");
 constexpr int kClusterFrom = 2048;
 constexpr int kListed = 1024;     // values that a CTA can list
 // few_survivors_kernel: the largest k, and the most values that it may find above its bound. Of 2048 shares, k = 256 of them hold the
-// 273 largest values on average, so twice k leaves room for values that lie together.
+// 273 largest values on average, so twice k leaves room for values that lie together. (Which calls take it: few_survivors below.)
 constexpr int kFewK = 256, kFound = 512;
 static_assert(2 * kFound <= kListed && kMaxCluster * kThreads <= 2 * kBins, "found values twice in the list, a key per thread in the bins");
 
@@ -583,7 +585,7 @@ multinomial_kernel(const float* __restrict__ logits, int n, const float* __restr
   multinomial_row(c, Row(const_cast<float*>(logits), n, c), uniforms, out, room, sh);
 }
 
-// for k above kFewK
+// where few_survivors does not hold
 __global__ void __launch_bounds__(kThreads, 4)
 top_k_kernel(float* __restrict__ logits, int n, int k) {
   __shared__ uint32_t bins[kBins];
@@ -820,6 +822,18 @@ few_survivors_kernel(float* __restrict__ logits, int n, const Chain ch) {
     for (int j = tid; j < kept; j += kThreads) row.l[sorted[j].x] = __int_as_float(sorted[j].y);
 }
 
+// Calls that few_survivors_kernel takes. Its time grows with k (each found value is an atomic, a further look at a share and a row of the ranking), and where k comes near the number of
+// shares that hold anything, most of a row is found and the general functions follow behind. What it saves are the launches of the chain, top-p's first, and reading long rows again. The
+// lines lie below the crossings measured at 1 and 64 rows of 300 to 151936 random values, its time against the launches', just within | at the next size beyond:
+// top-k alone: k = 24 | 48 at 300 values 0.85 | 1.2, 64 | 96 at 2048 1.0 | 1.17, 64 | 112 at 8192 0.87 | 1.03, 192 | 256 at 151936 0.80 | 1.12;
+// with the draw: 24 | 48 at 300 0.73 | 1.06, 80 | 112 at 1500 0.94 | 1.15, 80 | 112 at 2048 0.88 | 1.06, 96 | 160 at 8192 0.78 | 1.11, 192 | 256 at 65536 0.80 | 1.16;
+// with top-p as well: 32 | 80 at 300 0.51 | 1.21, 128 | 160 at 1500 0.84 | 1.10, 160 | 224 at 2048 0.78 | 1.17, 192 | 256 at 8192 0.76 | 1.04.
+bool few_survivors(int n, int k, float p, bool draw) {
+  const int shares = std::min((n + 3) / 4, (n < kClusterFrom ? 1 : kMaxCluster) * kThreads);
+  const int most = p < 1.0f ? std::min(9 * shares / 16, 160 + n / 256) : draw ? std::min(3 * shares / 8, 80 + n / 512) : std::min(3 * shares / 8, 64 + n / 1024);
+  return k > 0 && k < n && k <= std::min(most, kFewK);
+}
+
 // a row is a cluster of eight CTAs, or one CTA
 template <typename... P, typename... A>
 uint32_t launch_rows(void (*kern)(P...), int rows, int n, void* stream, A... args) {
@@ -858,7 +872,7 @@ uint32_t logismos_launch_top_k_f32(void* logits, int32_t rows, int32_t n, int32_
   lg::LaunchScope launch_scope_;
   if (rows < 0 || n < 0 || k < 0 || !logits) return lg::kInvalidValue;
   if (k == 0 || k >= n || rows == 0) return 0;
-  if (k <= kFewK) return launch_rows(few_survivors_kernel, rows, n, stream, (float*)logits, n, Chain{1.0f, k, 1.0f, 0.0f, nullptr, nullptr});
+  if (few_survivors(n, k, 1.0f, false)) return launch_rows(few_survivors_kernel, rows, n, stream, (float*)logits, n, Chain{1.0f, k, 1.0f, 0.0f, nullptr, nullptr});
   return launch_rows(top_k_kernel, rows, n, stream, (float*)logits, n, k);
 }
 
@@ -902,7 +916,7 @@ uint32_t logismos_launch_sample_chain_f32(void* logits, int32_t rows, int32_t n,
   lg::LaunchScope launch_scope_;
   if (rows < 0 || n < 0 || k < 0 || !logits || !out_u32 || (rows > 0 && n > 0 && !uniforms_f32)) return lg::kInvalidValue;
   if (rows == 0) return 0;
-  if (k > 0 && k <= kFewK && k < n) {
+  if (few_survivors(n, k, p, true)) {
     const float t = fmaxf(temperature, 1e-6f);
     return launch_rows(few_survivors_kernel, rows, n, stream, (float*)logits, n,
                        Chain{fabsf(t - 1.0f) < 1e-9f ? 1.0f : t, k, fminf(fmaxf(p, 0.0f), 1.0f), fminf(fmaxf(min_p, 0.0f), 1.0f), (const float*)uniforms_f32, (uint32_t*)out_u32});

@@ -124,7 +124,7 @@ _FUSED = {TemperatureScale: 0, TopK: 1, TopP: 2, MinP: 3}  # the places of a cha
 
 class DecodeChain:
     """chain.rs:33-76: processors in insertion order, then the sampler. Temperature, top-k, top-p and min-p in that order with a
-    multinomial draw run as one launch where k is at most 256, with the same results."""
+    multinomial draw are one call, and one launch where k is small for the row (at most 256), with the same results."""
 
     def __init__(self, sampler):
         self.processors, self.sampler = [], sampler
