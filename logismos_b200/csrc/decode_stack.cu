@@ -113,6 +113,26 @@ LG_DEVINL void receive(uint2 (&out)[N], uint32_t number, volatile int* abort_fla
   }
 }
 
+// The numbers have been through 32 bits: every word is zero again, as before the first launch. All CTAs meet, once in 2^32 layers.
+__device__ __noinline__ bool clear_words(Word* words, size_t n, uint32_t* met) {
+  __shared__ int s_ok;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) words[i] = 0;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const uint32_t until = (atomicAdd(met, 1u) / gridDim.x + 1) * gridDim.x;
+    s_ok = 0;
+#pragma unroll 1
+    for (uint32_t i = 0; i < kPolls && !s_ok; ++i) {
+      uint32_t v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(met) : "memory");
+      s_ok = (int)(v - until) >= 0;
+    }
+  }
+  __syncthreads();
+  return s_ok;
+}
+
 // what the CTA's weight slot stands for
 LG_DEVINL int weight_row(const StackPlan& p, int m, int cta, int slot) {
   if (m == kOut || m == kDown) return cta * p.out_rows + slot;
@@ -539,6 +559,7 @@ template <int R>
 __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_kernel(const __grid_constant__ Kernel kern) {
   __shared__ __align__(8) uint64_t s_bars[2 * kMats];
   __shared__ int s_abort;
+  __shared__ uint32_t s_before;  // launches before this one since the words were zero
   __shared__ float s_red[R * kMaxWarps];
   __shared__ StackLayer s_layer[2];  // this layer's and the next one's addresses
   __shared__ Mail s_mail;
@@ -570,6 +591,7 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
     s_mail.act = take((size_t)R * I / 2);
   }
   if (tid < kLayerWords) reinterpret_cast<uint64_t*>(s_layer)[tid] = layer_word(0);
+  if (tid == 0) s_before = *a.launches;
   const uint32_t parts = p.at_part;
   // the parts of warps that are not there are zero whenever sums are taken: what else goes to their place is cleared again
   auto clear_tail = [&](int n) {
@@ -577,6 +599,14 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
   };
   clear_tail(blockDim.x);
   __syncthreads();
+  if (s_before >= a.most_launches) {
+    const bool ok = clear_words(a.words, a.n_words, a.launches + 1);
+    if (tid == 0) {
+      s_before = 0;
+      if (!ok) s_abort = 1;
+    }
+    __syncthreads();
+  }
 
   // rows of this CTA and what they are, the same in every layer
   const int n_qkv = 16 * max(0, min(p.qkv_tiles, all_heads * (kDim / 16) - cta * p.qkv_tiles)), n_gu = 16 * max(0, min(p.gu_tiles, I / 8 - cta * p.gu_tiles)),
@@ -648,7 +678,7 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
   const uint32_t stage = smem_u32(smem) + p.at[kDown] + (uint32_t)(warp * kStage);
   const int block0 = cta < items && warp < p.att_warps && warp < s_item.count ? block_of(kern, s_item, warp) : -1;
   float4 gain = load4_now(s_layer[0].norm1 + 4 * tid);
-  uint32_t number = *a.launches * (uint32_t)a.n_layers;
+  uint32_t number = s_before * (uint32_t)a.n_layers;
 #pragma unroll 1
   for (int l = 0; l < a.n_layers; ++l) {
     const StackLayer& L = s_layer[l & 1];
@@ -816,7 +846,7 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
     }
   }
   // A CTA that has finished its down projection has seen results of all CTAs that take part, so they have read the count. (CTA 0 has rows of every matrix.)
-  if (cta == 0 && tid == 0) *a.launches += 1;
+  if (cta == 0 && tid == 0) *a.launches = s_before + 1;
   __syncthreads();
   if (s_abort) {
     // a wait expired: copies that may still be in flight land before the shared memory is released

@@ -46,6 +46,9 @@ int stack_chunk(const StackPlan& plan, const int32_t* ctx, int rows);
 bool stack_blocks_apart(const int32_t* tables, int max_blocks, const int32_t* ctx, int rows);
 // 64-bit words by which the CTAs of launches of up to d.rows rows pass on results; all zero before the first launch and after a failed one
 size_t stack_words(const StackDims& d);
+// Launches whose numbers, one per layer from 1 on, fit 32 bits. A model's count starts 64 short of it, so that the words are cleared soon and not after weeks.
+inline uint32_t stack_most_launches(int n_layers) { return 0xffffffffu / (uint32_t)(n_layers > 0 ? n_layers : 1); }
+inline uint32_t stack_first_count(int n_layers) { return stack_most_launches(n_layers) > 64 ? stack_most_launches(n_layers) - 64 : 0; }
 
 struct StackArgs {
   StackDims d;
@@ -59,8 +62,10 @@ struct StackArgs {
   const int64_t* slots;
   const int *ctx, *tables;
   int max_blocks, n_pool_blocks, chunk;
-  unsigned long long* words;  // stack_words
-  uint32_t* launches;         // how many went before, with the words
+  unsigned long long* words;  // n_words = stack_words of the most rows
+  size_t n_words;
+  uint32_t* launches;         // how many went before since the words were zero; the CTAs that met to clear them
+  uint32_t most_launches;     // whose numbers fit 32 bits: the next one clears the words
   int* status;
 };
 uint32_t launch_decode_stack(const StackArgs& a, const StackPlan& plan, cudaStream_t stream);

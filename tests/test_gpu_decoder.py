@@ -224,7 +224,7 @@ def test_one_launch_with_warps_that_are_no_multiple_of_four(heads, kv, inter, n_
     qw, _ = quantize_weights(cfg, make_weights(cfg, 13))
     model = DecoderModel(cfg, qw, n_pool_blocks=300, max_blocks_per_seq=100, max_step_tokens=1536, max_step_seqs=4)
     rng, alloc = np.random.default_rng([heads, n_seqs]), BlockAllocator(300, 100, seed=2)
-    lens = [400, 1500, 20, 150]
+    lens = [400, 900, 20, 150]
     tables = np.stack([alloc.ensure(i, n + 1) for i, n in enumerate(lens)])
     for i, n in enumerate(lens):
         model.step(rng.integers(0, 520, n), [0], [n], tables[i:i + 1])
@@ -241,6 +241,39 @@ def test_one_launch_with_warps_that_are_no_multiple_of_four(heads, kv, inter, n_
                 lib.logismos_set_deterministic(0)
         for i in range(n_seqs):
             assert max_rel(out[0][0][i], out[1][0][i]) <= TOL and max_rel(out[0][1][i], out[1][1][i]) <= TOL, (first, i)
+    model.close()
+
+
+@pytest.mark.parametrize("before", [62, 63, 64, 65])
+def test_numbers_of_the_one_launch_start_again(before):
+    """The words that CTAs exchange carry numbers of 32 bits. A model's count starts 64 launches short of where they end: steps of one row up to there, then one of four rows, whose words
+    have not all been written before, and two more. Bound: as the tests against the oracle."""
+    from logismos_b200._lib import lib
+    cfg = dict(TINY, hidden=512, n_heads=4, n_kv_heads=2, intermediate=512, vocab=512, n_layers=3, max_pos=1024)
+    qw, _ = quantize_weights(cfg, make_weights(cfg, 9))
+    model = DecoderModel(cfg, qw, n_pool_blocks=128, max_blocks_per_seq=32, max_step_tokens=512, max_step_seqs=4)
+    rng, alloc = np.random.default_rng(4), BlockAllocator(128, 32, seed=2)
+    lens = [17, 300, 129, 64]
+    tables = np.stack([alloc.ensure(i, n + 1) for i, n in enumerate(lens)])
+    for i, n in enumerate(lens):
+        model.step(rng.integers(0, 512, n), [0], [n], tables[i:i + 1])
+
+    def step(rows, det):
+        lib.logismos_set_deterministic(det)
+        try:
+            model.step(list(range(rows)), lens[:rows], [1] * rows, tables[:rows])
+            assert (model.launches_last_step() <= 7) == (det == 0)
+            return model.last_logits().copy()
+        finally:
+            lib.logismos_set_deterministic(0)
+
+    want = step(4, 1)
+    for _ in range(before):
+        first = step(1, 0)
+    assert max_rel(first, want[:1]) <= TOL
+    for rows in (4, 1, 3):
+        got = step(rows, 0)
+        assert max_rel(got, want[:rows]) <= TOL, rows
     model.close()
 
 
