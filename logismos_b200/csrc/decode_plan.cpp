@@ -64,6 +64,10 @@ int stack_chunk(const StackPlan& plan, const int32_t* ctx, int rows) {
   return std::max(round_up(least, kTokens), kTokens * plan.att_warps);
 }
 
+bool stack_contexts(const StackPlan& plan, const int32_t* ctx, int rows) {
+  return (stack_chunk(plan, ctx, rows) / kTokens + plan.att_warps - 1) / plan.att_warps <= kMaxRounds;
+}
+
 bool stack_blocks_apart(const int32_t* tables, int max_blocks, const int32_t* ctx, int rows) {
   for (int r = 0; r < rows; ++r) {
     const int last = (ctx[r] - 1) / kTokens;

@@ -90,7 +90,7 @@ uint32_t run_device(Decoder* m, cudaStream_t s) {
   const bool few = !logismos_get_deterministic() && m->n_pre == 0 && lg::int4_rows_fit(T, std::max(H, I)) && !c.kv_turbo3;
   const lg::StackDims dims{H, I, c.n_heads, c.n_kv_heads, T};
   lg::StackPlan plan;
-  const bool stack = few && m->stack && lg::stack_plan(dims, lg::sm_count(), &plan) && lg::stack_blocks_apart(m->batch.tables, c.max_blocks_per_seq, m->batch.ctx, T);
+  const bool stack = few && m->stack && lg::stack_plan(dims, lg::sm_count(), &plan) && lg::stack_contexts(plan, m->batch.ctx, T) && lg::stack_blocks_apart(m->batch.tables, c.max_blocks_per_seq, m->batch.ctx, T);
   if (stack) {
     lg::StackArgs a{};
     a.d = dims;

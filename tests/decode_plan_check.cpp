@@ -49,6 +49,9 @@ static bool check(const StackDims& d, const StackPlan& p) {
     const int chunk = stack_chunk(p, &ctx, 1);
     if (chunk % kTokens || (ctx + chunk - 1) / chunk > p.max_chunks || p.max_chunks > kMaxChunks) return std::printf("chunks of %d tokens for %d\n", chunk, ctx), false;
   }
+  int ctx = 1;
+  while (stack_contexts(p, &ctx, 1)) ctx += kTokens;
+  if (ctx <= kMaxRounds * kTokens || stack_chunk(p, &ctx, 1) <= kMaxRounds * kTokens * p.att_warps) return std::printf("contexts end at %d tokens\n", ctx), false;
   return true;
 }
 

@@ -244,6 +244,31 @@ def test_one_launch_with_warps_that_are_no_multiple_of_four(heads, kv, inter, n_
     model.close()
 
 
+def test_long_contexts_of_many_key_heads_do_not_take_the_one_launch():
+    """Six key heads and four rows leave six chunks per context: a step at 1500 tokens needs 8 rounds of cache blocks and takes the one launch, at 3000 tokens 16 and does not. Bound:
+    as the tests against the oracle."""
+    from logismos_b200._lib import lib
+    cfg = dict(TINY, hidden=768, n_heads=6, n_kv_heads=6, intermediate=1024, vocab=512, max_pos=4096)
+    qw, _ = quantize_weights(cfg, make_weights(cfg, 5))
+    model = DecoderModel(cfg, qw, n_pool_blocks=512, max_blocks_per_seq=200, max_step_tokens=3072, max_step_seqs=4)
+    rng, alloc = np.random.default_rng(1), BlockAllocator(512, 200, seed=2)
+    tables = np.stack([alloc.ensure(i, n + 1) for i, n in enumerate((3000, 70, 33, 5))])
+    for i, n in enumerate((3000, 70, 33, 5)):
+        model.step(rng.integers(0, 512, n), [0], [n], tables[i:i + 1])
+    for ctx, one in ((1500, True), (3000, False)):
+        out = []
+        for det in (0, 1):
+            lib.logismos_set_deterministic(det)
+            try:
+                model.step([5, 6, 7, 8], [ctx, 70, 33, 5], [1] * 4, tables)
+                out.append(model.last_logits().copy())
+                assert (model.launches_last_step() <= 7) == (one and det == 0), (ctx, det, model.launches_last_step())
+            finally:
+                lib.logismos_set_deterministic(0)
+        assert max_rel(out[0], out[1]) <= TOL
+    model.close()
+
+
 @pytest.mark.parametrize("before", [62, 63, 64, 65])
 def test_numbers_of_the_one_launch_start_again(before):
     """The words that CTAs exchange carry numbers of 32 bits. A model's count starts 64 launches short of where they end: steps of one row up to there, then one of four rows, whose words
