@@ -93,18 +93,18 @@ struct HostRows {
           return e;
         }
       }
-      const int movers = parts == 1 ? 1 : (int)std::max(1u, std::min({(unsigned)kMovers, std::thread::hardware_concurrency(), (unsigned)((size_t)n * row / kAlone)}));
+      const int movers = parts == 1 ? 1 : (int)std::max(1u, std::min({(unsigned)kMovers, std::thread::hardware_concurrency(), (unsigned)(4 * (size_t)n * row / kAlone)}));  // a quarter of a MB each
       std::atomic<int> arrived{0};  // parts in the pinned buffer; negative: no more will come
       auto move_on = [&](int i, int w) {
         const size_t c0 = width * w / movers, c1 = width * (w + 1) / movers;
         for (int k = n * i / parts; k < n * (i + 1) / parts; ++k)
           std::memcpy(host_out + (size_t)order[r0 + k] * width + c0, pinned + (size_t)k * row + c0 * 4, (c1 - c0) * 4);
       };
-      auto touch = [&](int w) {  // the page faults of a range: all of it is written later
+      auto touch = [&](int w) {  // the page faults of a range
         const size_t c0 = width * w / movers, c1 = width * (w + 1) / movers;
         for (int k = 0; k < n; ++k) {
           volatile uint8_t* dst = reinterpret_cast<uint8_t*>(host_out + (size_t)order[r0 + k] * width + c0);
-          for (size_t at = 0; at < (c1 - c0) * 4; at += kPage) dst[at] = 0;
+          for (size_t at = 0; at < (c1 - c0) * 4; at += kPage) dst[at] = dst[at];  // (rows that do not arrive stay as they were)
         }
       };
       // A thread of its own for a range of columns. Only the calling one calls CUDA: a new thread stands on device 0 until it chooses another.

@@ -54,10 +54,20 @@ int main() {
   }
   g_no_pinned = false;
   g_fail_event = g_events + 2;  // a wait in the middle fails: the error comes back, no thread is left behind
-  std::vector<float> dev(64 * 32768), out(dev.size());
+  std::vector<float> dev(64 * 32768), out(dev.size() + 1, 0.1f);
   std::vector<int> order(64);
   for (int i = 0; i < 64; ++i) order[i] = i;
-  if (rows.copy(dev.data(), 64, 32768, order.data(), out.data(), nullptr) != cudaErrorLaunchFailure) return std::puts("a failed wait went unseen"), 1;
+  for (size_t i = 0; i < dev.size(); ++i) dev[i] = (float)(i % 16777213) + 1.0f;
+  // (from an address that is no multiple of a page, nor are its rows' ranges)
+  if (rows.copy(dev.data(), 64, 32768, order.data(), out.data() + 1, nullptr) != cudaErrorLaunchFailure) return std::puts("a failed wait went unseen"), 1;
+  for (size_t i = 0; i < dev.size(); ++i)
+    if (out[i + 1] != dev[i] && out[i + 1] != 0.1f) return std::printf("value %zu is neither what it was nor what was sent\n", i), 1;
+  if (out.back() != 0.1f) return std::puts("the last row came although its part did not"), 1;
+  for (int n : {8, 9, 10, 12, 15, 16, 17, 33}) {  // one to several threads, rows off a page
+    std::fill(out.begin(), out.end(), 0.1f);
+    if (rows.copy(dev.data(), n, 32767, order.data(), out.data() + 1, nullptr) != cudaSuccess) return std::puts("copy failed"), 1;
+    if (std::memcmp(out.data() + 1, dev.data(), (size_t)n * 32767 * 4) || out[0] != 0.1f || out[(size_t)n * 32767 + 1] != 0.1f) return std::printf("%d rows\n", n), 1;
+  }
   rows.release();
   if (g_foreign) return std::printf("%d of %d CUDA calls from other threads\n", g_foreign.load(), g_calls.load()), 1;
   return 0;
