@@ -53,8 +53,9 @@ struct Cfg {
 };
 
 // x / (1 + exp(-x)), a rounded division here and in int4_rows. LATENCY: the quotient by Markstein's correction (q + r * (x - q * d), IBM J. Res. Dev. 34,
-// 1990) in place of the operator, whose branches keep the quotients of a row from overlapping; the same bits but for 2 of 1.8e9 floats, which differ in the last. Where d or
-// x is infinite the remainder is NaN and the first quotient is the answer. For tiles of 128 columns, which calls of few rows take and whose last epilogue nothing hides: it took 4100 cycles
+// 1990), made twice, in place of the operator, whose branches keep the quotients of a row from overlapping. The bits are the operator's for every x (all 2^32
+// compared; corrected once, two differ in the last bit), so a row does not depend on the tile that its call takes. Where d or x is infinite the remainder is NaN
+// and the first quotient is the answer, as it is where nothing remains. For tiles of 128 columns, which calls of few rows take and whose last epilogue nothing hides: it took 4100 cycles
 // with the operator (17920 x 1536 at 17 rows 17.8 -> 15.7 us, 12288 x 2048 at 64 17.2 -> 15.7, with the early requests below). Larger tiles hide it behind the next tile's MMAs, and there the
 // additional operations cost more than the branches: 861 against 885 us for 17920 x 1536 at 20 thousand rows, by pairs.
 template <bool LATENCY>
@@ -66,8 +67,8 @@ LG_DEVINL float silu_f(float x) {
   d *= scale;
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(d));
-  const float q = x * r, rem = fmaf(-q, d, x), fixed = fmaf(rem, r, q);
-  return rem == rem ? fixed : q;
+  const float q = x * r, rem = fmaf(-q, d, x), once = fmaf(rem, r, q);
+  return fabsf(rem) > 0.0f ? fmaf(fmaf(-once, d, x), r, once) : q;
 }
 
 // eight bias values (the same for every lane); vec: the pointer is 16-byte aligned

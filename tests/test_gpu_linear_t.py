@@ -147,6 +147,46 @@ def test_swiglu_divides_with_rounding(m):
     assert ((got - ref).abs() <= (2 ** -8 + 2e-4) * ref.abs()).all(), (got[0, :8], ref[0, :8])
 
 
+def test_swiglu_does_not_depend_on_the_tile():
+    """Gates at which a quotient corrected once is not the rounded one, with up values that bring the last bit of the quotient into the bf16 result: adjacent floats around silu(g) times u
+    lie on two sides of a boundary of bf16. One row (tiles of 128 columns) against 40000 (of 256), bit for bit; every sum is of up to three bf16 parts and exact."""
+    f32 = np.float32
+
+    def parts(x):  # three bf16 values that add up to a float
+        out, rest = [], f32(x)
+        for _ in range(3):
+            out.append((np.atleast_1d(rest).view(np.uint32) & np.uint32(0xffff0000)).view(f32)[0])
+            rest = f32(rest - out[-1])
+        assert rest == 0
+        return out
+
+    rn = lambda v: float(torch.tensor(float(v)).to(torch.bfloat16))
+    cols = []
+    for bits in (0x3e609af2, 0x3e24a9bf):
+        g = np.array([bits], np.uint32).view(f32)[0]
+        s = f32(float(g) / (1.0 + np.exp(-float(g))))
+        for step in range(-4, 4):  # the device's exponential may move the quotient some units
+            lo = np.array([int(s.view(np.uint32)) + step], np.uint32).view(f32)[0]
+            hi, found = np.nextafter(lo, f32(1)), 0
+            for i in range(128):
+                u = f32(2 * (1 + (2 * i + 1) / 256) / (float(lo) + float(hi)))  # their product with u: about half way between two values of bf16
+                for v in (u, np.nextafter(u, f32(0)), np.nextafter(u, f32(99))):
+                    if found < 8 and rn(f32(lo * v)) != rn(f32(hi * v)):
+                        cols.append((g, v))
+                        found += 1
+            assert found, (bits, step)
+    n, k, m = 1024, 64, 40000
+    z = torch.zeros((n // 64, 2, 32, k))
+    for j in range(n // 2):
+        g, u = cols[j % len(cols)]
+        z[j // 32, 0, j % 32, 0:3] = torch.tensor(parts(g)); z[j // 32, 1, j % 32, 3:6] = torch.tensor(parts(u))
+    a = torch.zeros((m, k)); a[:, :6] = 1.0
+    a, w = a.to(DEV, torch.bfloat16), z.view(n, k).to(DEV, torch.bfloat16)
+    assert torch.equal(w.float().cpu(), z.view(n, k)) and tile_of(1, n, k, ops.EPI_SWIGLU)[0] == 128 and tile_of(m, n, k, ops.EPI_SWIGLU)[0] == 256
+    one, many = ops.linear_t(a[:1].contiguous(), w, swiglu=True), ops.linear_t(a, w, swiglu=True)
+    assert torch.equal(one.expand(m, -1), many)
+
+
 @pytest.mark.parametrize("m,n,k", [(800, 1536, 8960), (1024, 1536, 1536), (600, 2048, 8192)])
 def test_outputs_that_fill_half_the_chip_repeat(m, n, k):
     """Residual updates of middle size are one sum over k per element: the same bits every time, and those of 200 rows at a time, which
