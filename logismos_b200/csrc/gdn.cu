@@ -498,7 +498,7 @@ gdn_decode_fused_kernel(float* __restrict__ state, float* __restrict__ acc, int6
   }
 }
 
-// The same step for batches whose halves of heads do not all fit at once. What bounds it is the 128 KB of state per (sequence, head) that cross HBM; the
+// The same step for batches whose halves of heads do not all fit at once (where: logismos_launch_gdn_decode_from_acc). What bounds it is the 128 KB of state per (sequence, head) that cross HBM; the
 // kernel above leaves a part of that rate unused, since its CTAs load, compute and store in step and the last of its 3.5 waves (64 sequences of 16 heads) is half
 // empty. Here a CTA holds one whole head's state in shared memory (64 KB, three CTAs per SM, so 192 KB of reads in flight) and walks over several heads: every
 // thread copies, uses and writes back only its own 32 rows x 4 columns, so the copies of the next head start row by row behind the last use of this one and need no
@@ -688,7 +688,10 @@ extern "C" uint32_t logismos_launch_gdn_decode_from_acc(void* state, void* acc, 
   if (((uintptr_t)state & 15) || ((uintptr_t)acc & 15) || ((uintptr_t)o & 1) || ((uintptr_t)pair_count & 3)) return lg::kInvalidValue;
   const int64_t ctas = (int64_t)n_seqs * heads * PfCfg<2, 4>::kParts;
   if (ctas > 2147483647ll) return lg::kInvalidValue;
-  if (ctas > 4ll * lg::sm_count()) {  // more than the kernel of halves holds at once
+  // The walking kernel where it was the faster one inside decode steps (7 recurrent layers, us a layer with the rest of it, halves against walk; heads 8, 16, 32): more items than the
+  // kernel of halves holds at once (288 items 67.4, 67.5), up to nine an SM (1024 items of 64 sequences 97.1, 92.6; 512 of 64 76.8, 74.7; 1280 of 40 106.0, 103.4; 1408 of 44 110.8, 113.0; 2048 135.5, 135.2),
+  // and steps of more than 32 sequences, behind whose in-projection (64 rows wide) the halves gain less from their early start (512 items of 32 sequences 64.9, 69.2; 1024 of 32 84.0, 88.8).
+  if (n_seqs > 32 && ctas > 4ll * lg::sm_count() && ctas <= 18ll * lg::sm_count()) {
     constexpr size_t smem = (size_t)KD * VD * 4;
     const cudaError_t e = lg::allow_shared((const void*)gdn_decode_walk_kernel, smem);
     if (e != cudaSuccess) return (uint32_t)e;

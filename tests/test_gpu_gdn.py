@@ -160,7 +160,7 @@ def test_decode_from_the_workspace_equals_finish_then_recurrence():
     assert np.isfinite(to_np(o_b)).all()
 
 
-@pytest.mark.parametrize("T,heads", [(50, 6), (61, 8), (64, 16)])
+@pytest.mark.parametrize("T,heads", [(50, 6), (61, 8), (64, 16), (32, 16), (33, 10), (41, 32), (42, 32)])  # and the lines between the two kernels
 def test_decode_of_a_large_batch_equals_decode_in_parts(T, heads):
     """Batches whose CTAs walk over several heads (one, two and three heads per CTA) against the same sequences in calls small enough for one half of a head per CTA: outputs, states and the
     zeroed workspace bit for bit; state slots permuted, fresh sequences first, last and between."""
