@@ -160,7 +160,7 @@ def test_decode_from_the_workspace_equals_finish_then_recurrence():
     assert np.isfinite(to_np(o_b)).all()
 
 
-@pytest.mark.parametrize("T,heads", [(50, 6), (61, 8), (64, 16), (32, 16), (33, 10), (41, 32), (42, 32)])  # and the lines between the two kernels
+@pytest.mark.parametrize("T,heads", [(50, 6), (61, 8), (64, 16)])
 def test_decode_of_a_large_batch_equals_decode_in_parts(T, heads):
     """Batches whose CTAs walk over several heads (one, two and three heads per CTA) against the same sequences in calls small enough for one half of a head per CTA: outputs, states and the
     zeroed workspace bit for bit; state slots permuted, fresh sequences first, last and between."""
@@ -188,6 +188,12 @@ def test_decode_of_a_large_batch_equals_decode_in_parts(T, heads):
 
     for got, want in zip(run(T), run(8)):
         assert torch.equal(got, want) and bool(torch.isfinite(got.float()).all())
+
+
+@pytest.mark.parametrize("T,heads", [(32, 16), (33, 10), (41, 32), (42, 32)])
+def test_decode_at_the_lines_between_the_two_kernels_equals_decode_in_parts(T, heads):
+    """32 | 33 sequences, and the last batch of 32 heads whose CTAs walk | the next one."""
+    test_decode_of_a_large_batch_equals_decode_in_parts(T, heads)
 
 
 def test_both_kernel_shapes_agree_with_the_reference():

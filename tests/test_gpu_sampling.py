@@ -251,23 +251,19 @@ def test_top_p_of_long_rows_keeps_small_probabilities(n):
 
 
 def _apart(chain, x, u):
-    """The chain's processors one by one, top-k by the oracle (up to 256 it would be the launch under test again), and the draw from the uniforms u."""
+    """The chain's processors one by one and the draw from the uniforms u."""
     t = torch.from_numpy(x.copy()).to(DEV)
     for p in chain.processors:
-        if isinstance(p, S.TopK):
-            t = torch.from_numpy(np.stack([O.top_k(row, p.k) for row in t.cpu().numpy()])).to(DEV)
-        else:
-            p.process(t)
+        p.process(t)
     return t, S.MultinomialSampler(seed=1).sample(t, uniforms=u)
 
 
-@pytest.mark.parametrize("n,k", [(n, k) for n in (2, 5, 255, 300, 1500, 2047, 2048, 2050, 8195, 33001, 151936, 262150) for k in (1, 2, 50, 256, 257)] +
-                         # the largest k of the launch with top-p and without, and the next one
-                         [(300, 28), (300, 29), (300, 42), (300, 43), (2047, 83), (2047, 84), (2047, 144), (2047, 145), (2048, 84), (2048, 85), (2048, 168), (2048, 169), (33001, 144), (33001, 145)])
+@pytest.mark.parametrize("n", [2, 5, 255, 300, 1500, 2047, 2048, 2050, 8195, 33001, 151936, 262150])
+@pytest.mark.parametrize("k", [1, 2, 50, 256, 257])
 def test_a_chain_in_one_launch_leaves_what_its_processors_leave(n, k):
     """Temperature, top-k, top-p, min-p and draw as one launch against one launch each: the same survivors to the bit. Rows of random values, of few values (more ties
     at the cut than the launch lists), of one value, with fewer finite values than k, with NaN and infinities, with the largest values side by side, all -inf; rows that
-    start off a 16-byte boundary (odd n). k below, at and above the largest that the launch takes at a length. Draws may differ where both lie within 1e-5 of the draw
+    start off a 16-byte boundary (odd n). k below, at and above the largest that the launch takes. Draws may differ where both lie within 1e-5 of the draw
     in the survivors' cumulative mass (fp32 sums of at most 512 normalised masses in another order)."""
     rng = np.random.default_rng([n, k])
     x = (rng.standard_normal((9, n)) * 3.0).astype(np.float32)
@@ -297,6 +293,26 @@ def test_a_chain_in_one_launch_leaves_what_its_processors_leave(n, k):
         v = torch.rand(9, generator=S.MultinomialSampler(seed=5).gen, device=DEV, dtype=torch.float32)
         S.check(S.lib.logismos_launch_sample_chain_f32(S._p(got.copy_(torch.from_numpy(x))), 9, n, *chain._settings(), S._p(v), S._p(tokens), S._stream()), "sample_chain")
         assert torch.equal(stepped.view(torch.int32), ref.view(torch.int32)) and torch.equal(drawn, tokens)
+
+
+def _apart_by_the_oracle(chain, x, u):
+    """As _apart with top-k by the oracle: as a processor it would be the launch under test again where that takes its k."""
+    t = torch.from_numpy(x.copy()).to(DEV)
+    for p in chain.processors:
+        if isinstance(p, S.TopK):
+            t = torch.from_numpy(np.stack([O.top_k(row, p.k) for row in t.cpu().numpy()])).to(DEV)
+        else:
+            p.process(t)
+    return t, S.MultinomialSampler(seed=1).sample(t, uniforms=u)
+
+
+@pytest.mark.parametrize("n,k", [(n, k) for n in (2, 5, 255, 300, 1500, 2047, 2048, 2050, 8195, 33001, 151936, 262150) for k in (1, 2, 50, 256, 257)] +
+                         # the largest k of the launch with top-p and without, and the next one
+                         [(300, 28), (300, 29), (300, 42), (300, 43), (2047, 83), (2047, 84), (2047, 144), (2047, 145), (2048, 84), (2048, 85), (2048, 168), (2048, 169), (33001, 144), (33001, 145)])
+def test_a_chain_in_one_launch_keeps_the_top_k_of_the_oracle(n, k, monkeypatch):
+    """The test above, its rows and bounds, with the survivors of top-k from the oracle."""
+    monkeypatch.setitem(globals(), "_apart", _apart_by_the_oracle)
+    test_a_chain_in_one_launch_leaves_what_its_processors_leave(n, k)
 
 
 def test_chains_of_another_shape_run_one_launch_per_processor():
