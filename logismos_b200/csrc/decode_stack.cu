@@ -626,6 +626,12 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
       if (i >= 0 && !mbar_wait_sleep_warp(frees + 8u * m, (uint32_t)(l & 1), &s_abort)) break;
       go(first, i < 0 ? 0 : next);
     }
+    // The last CTA that comes here writes the count that the next launch finds: all have read this one's. (A CTA without a part in the step, at narrow widths, is
+    // waited for by nobody else. It would take a count that changed under it for a reason to clear the words.)
+    if (warp == warps && lane == 0) {
+      __threadfence();
+      if (atomicInc(a.launches + 2, gridDim.x - 1) == gridDim.x - 1) *a.launches = s_before + 1;
+    }
     __syncthreads();
     return;
   }
@@ -845,8 +851,6 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + kBringers), 1) decode_stack_
       give_back(kGateUp);
     }
   }
-  // A CTA that has finished its down projection has seen results of all CTAs that take part, so they have read the count. (CTA 0 has rows of every matrix.)
-  if (cta == 0 && tid == 0) *a.launches = s_before + 1;
   __syncthreads();
   if (s_abort) {
     // a wait expired: copies that may still be in flight land before the shared memory is released

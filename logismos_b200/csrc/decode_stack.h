@@ -55,6 +55,8 @@ size_t stack_words(const StackDims& d);
 inline uint32_t stack_most_launches(int n_layers) { return 0xffffffffu / (uint32_t)(n_layers > 0 ? n_layers : 1); }
 inline uint32_t stack_first_count(int n_layers) { return stack_most_launches(n_layers) > 64 ? stack_most_launches(n_layers) - 64 : 0; }
 
+constexpr size_t kStackCounts = 2;  // words of 64 bits for the three counts behind the others
+
 struct StackArgs {
   StackDims d;
   const StackLayer* layers;
@@ -69,7 +71,7 @@ struct StackArgs {
   int max_blocks, n_pool_blocks, chunk;
   unsigned long long* words;  // n_words = stack_words of the most rows
   size_t n_words;
-  uint32_t* launches;         // how many went before since the words were zero; the CTAs that met to clear them
+  uint32_t* launches;         // how many went before since the words were zero; then the CTAs that met to clear them; then those of this launch that have read the first count
   uint32_t most_launches;     // whose numbers fit 32 bits: the next one clears the words
   int* status;
 };

@@ -99,7 +99,7 @@ uint32_t run_device(Decoder* m, cudaStream_t s) {
     a.cos = (const float*)m->cos.p; a.sin = (const float*)m->sin.p; a.positions = (const int*)m->pos.p; a.max_pos = c.max_pos; a.slots = (const int64_t*)m->slots.p;
     a.ctx = (const int*)m->dec_ctx.p; a.tables = (const int*)m->dec_tables.p; a.max_blocks = c.max_blocks_per_seq; a.n_pool_blocks = c.n_pool_blocks;
     a.chunk = lg::stack_chunk(plan, m->batch.ctx, T);
-    a.words = (unsigned long long*)m->stack_words.p; a.n_words = m->stack_words_bytes / 8 - 1; a.launches = (uint32_t*)(a.words + a.n_words);
+    a.words = (unsigned long long*)m->stack_words.p; a.n_words = m->stack_words_bytes / 8 - lg::kStackCounts; a.launches = (uint32_t*)(a.words + a.n_words);
     a.most_launches = lg::stack_most_launches(c.n_layers); a.status = (int*)st;
     LG_TRY(lg::launch_decode_stack(a, plan, s), "layers of a decode step of few rows");
     m->launches += 1;
@@ -266,10 +266,10 @@ uint32_t lg_decoder_create(int32_t device, const lg_decoder_config_t* cfg, const
        m->cu_prefill.alloc((S + 1) * 4) && m->last_idx.alloc(S * 4) && m->dec_ctx.alloc(S * 4) && m->dec_tables.alloc(S * MB * 4) &&
        m->dec_chunks.alloc((S + 1) * 4) && m->pre_kv.alloc(S * 4) &&
        m->dec_scratch.alloc(logismos_paged_decode_scratch_bytes((int32_t)m->max_chunks, c.n_heads, m->head_dim)) &&
-       m->stack_words.alloc(m->stack_words_bytes = 8 * (1 + lg::stack_words({(int)H, (int)I, c.n_heads, c.n_kv_heads, lg::kFewRows})));
+       m->stack_words.alloc(m->stack_words_bytes = 8 * (lg::kStackCounts + lg::stack_words({(int)H, (int)I, c.n_heads, c.n_kv_heads, lg::kFewRows})));
   ok = ok && cudaMemset(m->stack_words.p, 0, m->stack_words_bytes) == cudaSuccess;
   const uint32_t count = lg::stack_first_count(c.n_layers);
-  ok = ok && cudaMemcpy((char*)m->stack_words.p + m->stack_words_bytes - 8, &count, 4, cudaMemcpyHostToDevice) == cudaSuccess;
+  ok = ok && cudaMemcpy((char*)m->stack_words.p + m->stack_words_bytes - 8 * lg::kStackCounts, &count, 4, cudaMemcpyHostToDevice) == cudaSuccess;
   if (ok) {
     std::vector<lg::StackLayer> t((size_t)c.n_layers);
     auto mat = [](const QMat& q) { return lg::StackMat{(const uint8_t*)q.codes.p, (const __half*)q.scales.p}; };

@@ -302,6 +302,29 @@ def test_numbers_of_the_one_launch_start_again(before):
     model.close()
 
 
+def test_numbers_start_again_where_some_ctas_have_no_part():
+    """Two heads and one row: 18 of 148 CTAs have no weight rows, no chunk and nothing to put together. They read the count of launches and clear words with the others. Steps over the point
+    where the numbers start again and beyond. Bound: as the tests against the oracle."""
+    from logismos_b200._lib import lib
+    cfg = dict(TINY, hidden=256, n_heads=2, n_kv_heads=1, intermediate=256, vocab=512, n_layers=2, max_pos=1024)
+    qw, _ = quantize_weights(cfg, make_weights(cfg, 9))
+    model = DecoderModel(cfg, qw, n_pool_blocks=64, max_blocks_per_seq=32, max_step_tokens=512, max_step_seqs=4)
+    rng, alloc = np.random.default_rng(4), BlockAllocator(64, 32, seed=2)
+    tables = np.stack([alloc.ensure(0, 200)])
+    model.step(rng.integers(0, 512, 190), [0], [190], tables)
+    out = []
+    for det in [1] + 100 * [0]:
+        lib.logismos_set_deterministic(det)
+        try:
+            model.step([7], [190], [1], tables)
+            assert (model.launches_last_step() <= 7) == (det == 0)
+            out.append(model.last_logits().copy())
+        finally:
+            lib.logismos_set_deterministic(0)
+        assert max_rel(out[-1], out[0]) <= TOL, len(out)
+    model.close()
+
+
 def test_deterministic_switch_keeps_a_row_independent_of_its_step():
     """With the switch on, a sequence's decode steps have the same bits alone and beside 3, 4 and 29 others: the same projections and the
     same pieces of its context of 1000 tokens."""
