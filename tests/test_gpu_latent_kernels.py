@@ -254,6 +254,13 @@ def test_latent_decode_at_page_tile_and_chunk_borders(heads, rank, chunk):
         assert row_rel(got[i], latent_attend(q[i].astype(np.float64), c, 1.0 / rank)) <= TOL, LENS[i]
 
 
+@pytest.mark.parametrize("heads,rank", [(20, 128), (40, 128), (16, 256), (20, 256), (17, 512), (32, 512), (8, 640), (20, 640), (40, 640), (7, 1024)])
+@pytest.mark.parametrize("chunk", [0, 64])
+def test_latent_decode_of_ranks_that_fill_a_kernel(heads, rank, chunk):
+    """Ranks that are known at compile time, at the numbers of heads that the test above does not have them at. Its inputs and bounds."""
+    test_latent_decode_at_page_tile_and_chunk_borders(heads, rank, chunk)
+
+
 @pytest.mark.parametrize("heads,rank", [(1, 64), (7, 192), (4, 1024)])
 def test_latent_attention_f32(heads, rank):
     rng = np.random.default_rng(rank)
