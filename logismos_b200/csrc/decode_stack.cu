@@ -2,8 +2,11 @@
 //
 // Such a step is 28 layers x 26 MB of weights, 4 us a layer from HBM; as six launches a layer it took 42 us, nearly all of it starts of launches,
 // dependencies and first loads (int4_rows.cu has the launches); here 24. Device time of a step at contexts of 1200, one / two / three / four rows: 0.68 / 0.78 /
-// 0.86 / 0.93 ms against 1.20 / 1.28 / 1.45 / 1.55; at 300 and at 8000 the ratio is the same (1.5 to 1.8). What is left of a layer's 44 thousand cycles is six exchanges
-// between all SMs of some 3000 each, the products of gate and up (5000) and down (4800), which the unpacking of int4 on the ALU pipe bounds, and the attention.
+// 0.86 / 0.93 ms against 1.20 / 1.28 / 1.45 / 1.55; at 300 and at 8000 the ratio is the same (1.5 to 1.8). What is left of a layer, one row at 1200 tokens, by clock stamps of
+// thread 0 of every CTA (which cost 5 %; 45 thousand cycles a layer with them): q, k, v 7100 (2500 until the stream's words are there, norm 1400, products 1900, sums and rotation 1300);
+// 12900 from there until the merged heads are (3600 the attention of a CTA that has a chunk, the rest two exchanges and the merge); output 3600; gate and up 12700 (2700 until the words are there,
+// norm and products 7800, sums and SwiGLU 2200); down 8800 (2200, 5300, 1300). So an exchange between all SMs takes 2100 to 2700 cycles, and there are six; the products of
+// gate, up and down are bound by the unpacking of int4 on the ALU pipe. The step holds every SM: what other streams have for the GPU waits until it is over.
 //
 // One CTA per SM stays for the whole step. What an SM needs of a layer's weights (190 KB) fits its shared memory, so each matrix has a place there and the next
 // layer's copy (cp.async.bulk, a row at a time, rows 16 bytes apart modulo the banks, issued by a warp of its own) starts as soon as the products have used

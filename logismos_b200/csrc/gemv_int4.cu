@@ -835,9 +835,10 @@ extern "C" uint32_t logismos_launch_gemv_int4_g32_f32(const void* codes, const v
 // weight stream) and walks k serially per row tile, so few long rows leave most SMs idle; the
 // tensor-core kernel keeps the activations in one operand tile and splits k over the CTAs. Measured
 // crossovers (time per launch, weights from HBM): above 16 rows always; k >= 3 n at every batch
-// (1536 x 8960: 10.9 against 19.9 us at one row, 58 us at 16); 8 to 16 rows up to n = 16384 (7.8 against
-// 9.1 / 18.6 us for 1536 x 1536). The vocabulary-sized matrices stay on the GEMV up to 16 rows (55
-// against 67 us).
+// (1536 x 8960: 8.2 against 20.4 us at one row, 58 us at 16); 8 to 16 rows up to n = 16384 (5.9 against
+// 10.0 / 19.8 us for 1536 x 1536). The vocabulary-sized matrices stay on the GEMV up to 16 rows (33 against
+// 52 us at 8 rows of 151936 x 1536, 55 against 56 at 16). Since the tensor-core kernel unpacks faster it is ahead at 1 to 4
+// rows of small matrices too (5.7 against 6.7 to 8.3 us for 1536 x 1536); the lines are those of its former times.
 extern "C" int32_t logismos_skinny_int4_route(int32_t batch, int32_t n, int32_t k) {
   if ((k % 256) != 0 || (n % 4) != 0 || batch < 1 || batch > 64) return 0;
   if (batch > 16) return 1;

@@ -1,5 +1,5 @@
-// int4 group-32 projections of one to four rows, for decode steps of that many sequences: the hybrid decoder's, and the decoder's at widths that
-// decode_stack.cu does not take.
+// int4 group-32 projections of one to four rows, for decode steps of that many sequences: the hybrid decoder's, and the decoder's where
+// decode_stack.cu does not take a step (its width, long contexts of many key heads, blocks that sequences share).
 //
 // What bounds them is not the 1 to 16 MB of a matrix (0.2 to 2.4 us from HBM) but the length of a launch: start, dependency,
 // one round of latency to memory, a warp's own chain of instructions, the sum over k. The fused-dequant tcgen05 kernel takes 7.6 us
