@@ -325,6 +325,29 @@ def test_numbers_start_again_where_some_ctas_have_no_part():
     model.close()
 
 
+def test_one_launch_steps_replay_from_a_graph():
+    """A step's device work captured in a CUDA graph: the layers as one launch count their launches on the device, so each replay is the step again, bit for bit, also where the numbers
+    of the words start again."""
+    import torch
+    cfg = dict(TINY, hidden=512, n_heads=4, n_kv_heads=2, intermediate=512, vocab=512, n_layers=3, max_pos=1024)
+    qw, _ = quantize_weights(cfg, make_weights(cfg, 9))
+    model = DecoderModel(cfg, qw, n_pool_blocks=64, max_blocks_per_seq=32, max_step_tokens=512, max_step_seqs=4)
+    rng, alloc = np.random.default_rng(4), BlockAllocator(64, 32, seed=2)
+    tables = np.stack([alloc.ensure(i, n + 1) for i, n in enumerate((300, 17))])
+    for i, n in enumerate((300, 17)):
+        model.step(rng.integers(0, 512, n), [0], [n], tables[i:i + 1])
+    model.step([7, 9], [300, 17], [1, 1], tables)
+    want, stream, graph = model.last_logits().copy(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        model.replay_device(torch.cuda.current_stream().cuda_stream)
+    assert model.launches_last_step() <= 7
+    for _ in range(80):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert model.device_status() == 0 and np.array_equal(model.last_logits(), want)
+    model.close()
+
+
 def test_deterministic_switch_keeps_a_row_independent_of_its_step():
     """With the switch on, a sequence's decode steps have the same bits alone and beside 3, 4 and 29 others: the same projections and the
     same pieces of its context of 1000 tokens."""
