@@ -187,6 +187,25 @@ def test_swiglu_does_not_depend_on_the_tile():
     assert torch.equal(one.expand(m, -1), many)
 
 
+def test_swiglu_of_extreme_gates_does_not_depend_on_the_tile():
+    """Gates whose exponential overflows, vanishes or is near 2^100 and 2^126, zeros, the smallest and largest values, infinities, NaN: one row (tiles of 128 columns) against 40000 (of 256),
+    bit for bit."""
+    ln2 = float(np.log(2.0))
+    gates = [0.0, -0.0, 1e-38, -1e-38, 1e-30, -1e-30, 3e38, -3e38, float("inf"), float("-inf"), float("nan"), 88.5, -88.5, 100.0, -100.0]
+    gates += [-ln2 * e + d for e in (63, 64, 99, 100, 101, 125, 126, 127, 128) for d in (-0.5, 0.0, 0.5)]
+    gates += np.linspace(-110.0, 110.0, 512 - len(gates)).tolist()
+    n, k, m = 1024, 64, 40000
+    g = torch.tensor(gates, dtype=torch.float32).to(torch.bfloat16).float()
+    z = torch.zeros((n // 64, 2, 32, k))
+    z[:, 0, :, 0] = g.view(16, 32); z[:, 1, :, 1] = 1.0
+    a = torch.zeros((m, k)); a[:, :2] = 1.0
+    a, w = a.to(DEV, torch.bfloat16), z.view(n, k).to(DEV, torch.bfloat16)
+    assert tile_of(1, n, k, ops.EPI_SWIGLU)[0] == 128 and tile_of(m, n, k, ops.EPI_SWIGLU)[0] == 256
+    one, many = ops.linear_t(a[:1].contiguous(), w, swiglu=True), ops.linear_t(a, w, swiglu=True)
+    nan = one.isnan()
+    assert torch.equal(nan.expand(m, -1), many.isnan()) and torch.equal(torch.where(nan, 0.0, one).view(torch.int16).expand(m, -1), torch.where(nan, 0.0, many).view(torch.int16))
+
+
 @pytest.mark.parametrize("m,n,k", [(800, 1536, 8960), (1024, 1536, 1536), (600, 2048, 8192)])
 def test_outputs_that_fill_half_the_chip_repeat(m, n, k):
     """Residual updates of middle size are one sum over k per element: the same bits every time, and those of 200 rows at a time, which
