@@ -7,6 +7,9 @@
 #include <thread>
 #include <vector>
 
+#include <sys/mman.h>
+#include <sys/resource.h>
+
 #include "model_util.h"
 
 static std::thread::id g_caller;
@@ -70,6 +73,19 @@ int main() {
     std::fill(out.begin(), out.end(), 0.1f);
     if (rows.copy(dev.data(), n, 32767, order.data(), out.data() + 1, nullptr) != cudaSuccess) return std::puts("copy failed"), 1;
     if (std::memcmp(out.data() + 1, dev.data(), (size_t)n * 32767 * 4) || out[0] != 0.1f || out[(size_t)n * 32767 + 1] != 0.1f) return std::printf("%d rows\n", n), 1;
+  }
+  {  // a fresh destination costs one fault a page: reading a page ahead of the first write to it makes two of it, the second one with a flush on every core
+    const size_t bytes = dev.size() * 4, pages = bytes / 4096;
+    float* fresh = (float*)mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (fresh == MAP_FAILED) return std::puts("no memory"), 1;
+    madvise(fresh, bytes, MADV_NOHUGEPAGE);
+    rusage before, after;
+    getrusage(RUSAGE_SELF, &before);
+    if (rows.copy(dev.data(), 64, 32768, order.data(), fresh, nullptr) != cudaSuccess) return std::puts("copy failed"), 1;
+    getrusage(RUSAGE_SELF, &after);
+    if (std::memcmp(fresh, dev.data(), bytes)) return std::puts("rows of a fresh destination"), 1;
+    munmap(fresh, bytes);
+    if ((size_t)(after.ru_minflt - before.ru_minflt) > pages + pages / 2) return std::printf("%ld faults for %zu pages\n", after.ru_minflt - before.ru_minflt, pages), 1;
   }
   rows.release();
   if (g_foreign) return std::printf("%d of %d CUDA calls from other threads\n", g_foreign.load(), g_calls.load()), 1;
