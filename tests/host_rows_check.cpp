@@ -74,6 +74,17 @@ int main() {
     if (rows.copy(dev.data(), n, 32767, order.data(), out.data() + 1, nullptr) != cudaSuccess) return std::puts("copy failed"), 1;
     if (std::memcmp(out.data() + 1, dev.data(), (size_t)n * 32767 * 4) || out[0] != 0.1f || out[(size_t)n * 32767 + 1] != 0.1f) return std::printf("%d rows\n", n), 1;
   }
+  for (int n : {9, 15, 16}) {  // a destination that is fresh, and the same one again
+    const size_t bytes = (size_t)n * 32768 * 4;
+    float* fresh = (float*)mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (fresh == MAP_FAILED) return std::puts("no memory"), 1;
+    for (int again = 0; again < 2; ++again) {
+      if (lgm::HostRows::there(fresh, 32768, order.data(), n) != (again == 1)) return std::puts("pages"), 1;
+      for (float& v : dev) v += 1.0f;
+      if (rows.copy(dev.data(), n, 32768, order.data(), fresh, nullptr) != cudaSuccess || std::memcmp(fresh, dev.data(), bytes)) return std::printf("%d rows, %d\n", n, again), 1;
+    }
+    munmap(fresh, bytes);
+  }
   {  // a fresh destination costs one fault a page: reading a page ahead of the first write to it makes two of it, the second one with a flush on every core
     const size_t bytes = dev.size() * 4, pages = bytes / 4096;
     float* fresh = (float*)mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
